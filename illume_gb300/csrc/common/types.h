@@ -86,12 +86,15 @@ struct DevMesh {
   int pad[2];
 };
 
-struct DevInstance {
+// 128 bytes on a 16-byte boundary, read as 16-byte words: the box, mesh and material in two
+// loads, a matrix in three.
+struct alignas(16) DevInstance {
   float inv[12];                // world -> object rows
   float trans_inv[12];          // normal matrix rows
   float lo[3], hi[3];           // world-space bounds (padded)
   int mesh, material;
 };
+static_assert(sizeof(DevInstance) == 128, "instance record must be 128 bytes");
 
 struct DevSphere { float cx, cy, cz, r; int material; int pad[3]; };
 

@@ -44,8 +44,9 @@ __device__ __forceinline__ int event_class(const WaveBuffers& w, const JobDesc& 
 // shared counter (counters[44 + parity]) instead of a fixed grid stride, so that warps
 // whose rays finish early take over the remaining work.
 // PS, NF (4-wide only): see traverse_bvh4_ww.
+// ISECT: the triangle test, or -1 to take it from the knobs.
 template <int KIND, bool COUNT, int MINB = 1, bool OPT = false, bool WW = false, bool PS = false, bool NF = false,
-          bool FR = false, bool SI = false>
+          bool FR = false, bool SI = false, int ISECT = -1>
 __global__ void __launch_bounds__(128, MINB) k_trace(WaveBuffers w, RenderKnobs k, int bounce) {
   const int it = pass_iteration(w, bounce);
   const int parity = it & 1;
@@ -79,8 +80,8 @@ __global__ void __launch_bounds__(128, MINB) k_trace(WaveBuffers w, RenderKnobs 
     const SceneView& sc = J.sc;
     VisitCount vc;
     const HitRecord h =
-        closest_hit<KIND, COUNT, OPT, WW, false, PS, NF, FR, SI>(sc, v3(qo.x, qo.y, qo.z), v3(qd.x, qd.y, qd.z), k.isect,
-                                                         stack, &vc);
+        closest_hit<KIND, COUNT, OPT, WW, false, PS, NF, FR, SI, ISECT>(sc, v3(qo.x, qo.y, qo.z), v3(qd.x, qd.y, qd.z),
+                                                                k.isect, stack, &vc);
     if (COUNT) {
       my_nodes += vc.nodes;
       my_tris += vc.tris;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_refill(WaveBuffers w, RenderKn
 // radiance when nothing lies within the ray's maximum distance. Occlusion needs no
 // closest hit, so the traversal stops at the first hit (binary and 4-wide layouts);
 // warps take 32 rays at a time from a counter (counters[48 + parity]).
-template <int KIND>
+template <int KIND, int ISECT = -1>
 __global__ void __launch_bounds__(128, 8) k_shadow(WaveBuffers w, RenderKnobs k, int bounce) {
   const int parity = pass_iteration(w, bounce) & 1;
   const int n = w.counters[46 + parity];
@@ -270,8 +271,8 @@ __global__ void __launch_bounds__(128, 8) k_shadow(WaveBuffers w, RenderKnobs k,
     const SceneView& sc = w.jobs[job].sc;
     VisitCount vc;
     const HitRecord h =
-        closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, KIND != BVH_WIDE8, false, KIND == BVH_WIDE4>(
-            sc, v3(so.x, so.y, so.z), v3(sd.x, sd.y, sd.z), k.isect, stack, &vc, sd.w);
+        closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, KIND != BVH_WIDE8, false, KIND == BVH_WIDE4, KIND == BVH_WIDE4,
+                    false, ISECT>(sc, v3(so.x, so.y, so.z), v3(sd.x, sd.y, sd.z), k.isect, stack, &vc, sd.w);
     if (vc.dropped) atomicOr(w.counters + kCounterStackDrops, 1);
     if (h.geom == -1) {
       float4* c = w.contrib + __float_as_int(sv.w);
@@ -463,13 +464,19 @@ __global__ void __launch_bounds__(128) k_trace_hook(SceneView sc, const float4* 
 //   loaded by per-ray byte offsets, traversal stack in local memory (the default); 1 =
 //   four compare-swaps instead of five in the child ordering; 2 = lo and hi planes
 //   loaded and selected per child box; 3 = 6 blocks per SM (at most 80 registers).
+// The default 4-wide kernel is compiled once for the Moller-Trumbore test alone: without
+// the watertight test's six shear registers it spills nothing (132 / 368 bytes of spill
+// stores / loads otherwise). Traversal scene, 1024x1024, one 32-sample pass: 6.67 -> 6.51
+// ms of trace; Cornell box 256x256 at 64 samples: 0.61 -> 0.55 ms per pass. An instance
+// for the watertight test alone still spills 100 bytes and was 1.5% slower on 16 meshes
+// of 125k triangles (5.93 -> 6.01 ms), so that test stays in the general kernel.
 const void* trace_kernel_ptr(int bvh_kind, int variant) {
   if (bvh_kind == BVH_WIDE4) {
     if (variant == 1) return (const void*)k_trace<BVH_WIDE4, false, 8, true, false, true, true>;
     if (variant == 2) return (const void*)k_trace<BVH_WIDE4, false, 8, true>;
     if (variant == 3) return (const void*)k_trace<BVH_WIDE4, false, 6, true, false, false, true>;
     if (variant == 4) return (const void*)k_trace<BVH_WIDE4, false, 8, true, false, false, true>;
-    return (const void*)k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true>;
+    return (const void*)k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true, ISECT_MT>;
   }
   if (bvh_kind == BVH_WIDE8) {
     if (variant == 2) return (const void*)k_trace<BVH_WIDE8, false>;
@@ -499,7 +506,10 @@ void launch_trace(const WaveBuffers& w, const RenderKnobs& k, int bounce, int gr
       else k_trace<BVH_WIDE4, false, 8, true, false, false, true><<<grid, 128, 0, st>>>(w, k, bounce);
     } else {
       if (count_visits) k_trace<BVH_WIDE4, true, 8, true, false, false, true, true, true><<<grid, 128, 0, st>>>(w, k, bounce);
-      else k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true><<<grid, 128, 0, st>>>(w, k, bounce);
+      else if (k.isect == ISECT_MT)
+        k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true, ISECT_MT><<<grid, 128, 0, st>>>(w, k, bounce);
+      else
+        k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true><<<grid, 128, 0, st>>>(w, k, bounce);
     }
     return;
   }
@@ -541,12 +551,13 @@ void launch_trace(const WaveBuffers& w, const RenderKnobs& k, int bounce, int gr
 }
 
 const void* shadow_kernel_ptr(int bvh_kind) {
-  if (bvh_kind == BVH_WIDE4) return (const void*)k_shadow<BVH_WIDE4>;
+  if (bvh_kind == BVH_WIDE4) return (const void*)k_shadow<BVH_WIDE4, ISECT_MT>;
   return bvh_kind == BVH_WIDE8 ? (const void*)k_shadow<BVH_WIDE8> : (const void*)k_shadow<BVH_BINARY>;
 }
 
 void launch_shadow(const WaveBuffers& w, const RenderKnobs& k, int bounce, int grid, cudaStream_t st) {
-  if (k.bvh_kind == BVH_WIDE4) k_shadow<BVH_WIDE4><<<grid, 128, 0, st>>>(w, k, bounce);
+  if (k.bvh_kind == BVH_WIDE4 && k.isect == ISECT_MT) k_shadow<BVH_WIDE4, ISECT_MT><<<grid, 128, 0, st>>>(w, k, bounce);
+  else if (k.bvh_kind == BVH_WIDE4) k_shadow<BVH_WIDE4><<<grid, 128, 0, st>>>(w, k, bounce);
   else if (k.bvh_kind == BVH_WIDE8) k_shadow<BVH_WIDE8><<<grid, 128, 0, st>>>(w, k, bounce);
   else k_shadow<BVH_BINARY><<<grid, 128, 0, st>>>(w, k, bounce);
 }
