@@ -173,6 +173,8 @@ int Engine::init(Context* c, int nrows, int ncap, const RenderKnobs& k, std::str
   grid_shade = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant), 128, ctx->device);
   grid_shadow = kernel_grid_blocks(shadow_kernel_ptr(knobs.bvh_kind), 128, ctx->device);
   grid_shade_nee = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant, true), 128, ctx->device);
+  grid_paths = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, false), 128, ctx->device);
+  grid_paths_nee = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, true), 128, ctx->device);
   return ILLUME_OK;
 }
 
@@ -279,8 +281,13 @@ int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
       launch_iteration(side, cond, true, depth, nee);
     });
   }
+  if (path_pass(depth)) {
+    launch_paths(w, knobs, -1, depth, 0, nee ? grid_paths_nee : grid_paths, st, nee);
+    return ILLUME_OK;
+  }
   launch_raygen(w, grid_raygen, st);
   for (int b = 0; b < depth; ++b) {
+    if (hand_over(b)) launch_paths(w, knobs, b, depth, kPathTail, nee ? grid_paths_nee : grid_paths, st, nee);
     launch_trace(w, knobs, b, grid_trace, st);
     launch_shade(w, knobs, b, nee ? grid_shade_nee : grid_shade, st, nee);
     if (nee) launch_shadow(w, knobs, b, grid_shadow, st);
@@ -307,7 +314,7 @@ int Engine::run_interleaved(int depth, cudaEvent_t wait_ev, cudaEvent_t record_e
     const int s = ensure_shadow(&err);
     if (s != ILLUME_OK) { set_error(err); return s; }
   }
-  const int key = 2 * depth + (nee ? 1 : 0);
+  const int key = graph_key(depth, nee);
   auto it = head_graphs.find(key);
   if (it == head_graphs.end()) {
     cudaGraphExec_t exec = nullptr;
@@ -327,11 +334,12 @@ int Engine::run_interleaved(int depth, cudaEvent_t wait_ev, cudaEvent_t record_e
   if (wait_ev) ILLUME_CUDA_TRY(cudaStreamWaitEvent(stream, wait_ev, 0));
   ILLUME_CUDA_TRY(cudaGraphLaunch(acc_graph, stream));
   if (record_ev) ILLUME_CUDA_TRY(cudaEventRecord(record_ev, stream));
+  const int pass_launches = launches_per_pass(depth, nee);
   advance_mirror();
   passes += 1;
   if (!regen) {
-    launches += launches_per_pass(depth, nee);
-    ctx->launches += launches_per_pass(depth, nee);
+    launches += pass_launches;
+    ctx->launches += pass_launches;
   }
   return ILLUME_OK;
 }
@@ -349,7 +357,7 @@ int Engine::run(int npasses, int depth) {
     const int s = ensure_shadow(&err);
     if (s != ILLUME_OK) { set_error(err); return s; }
   }
-  const int key = 2 * depth + (nee ? 1 : 0);
+  const int key = graph_key(depth, nee);
   auto it = graphs.find(key);
   if (it == graphs.end()) {
     cudaGraphExec_t exec = nullptr;
@@ -357,14 +365,15 @@ int Engine::run(int npasses, int depth) {
     if (s != ILLUME_OK) return s;
     it = graphs.emplace(key, exec).first;
   }
+  const int pass_launches = launches_per_pass(depth, nee);   // one graph, whatever the passes' sizes
   for (int i = 0; i < npasses; ++i) {
     ILLUME_CUDA_TRY(cudaGraphLaunch(it->second, st));
     advance_mirror();
   }
   passes += npasses;
   if (!regen) {
-    launches += (long long)npasses * launches_per_pass(depth, nee);
-    ctx->launches += (long long)npasses * launches_per_pass(depth, nee);
+    launches += (long long)npasses * pass_launches;
+    ctx->launches += (long long)npasses * pass_launches;
   }
   return ILLUME_OK;
 }

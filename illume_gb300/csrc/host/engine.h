@@ -35,9 +35,10 @@ struct Engine {
   WaveBuffers w{};
   std::vector<JobDesc> mirror;   // the table as the device has it after the launched passes
   int grid_trace = 0, grid_shade = 0, grid_raygen = 0, grid_acc = 0, grid_shadow = 0, grid_shade_nee = 0;
+  int grid_paths = 0, grid_paths_nee = 0;
   cudaStream_t stream = nullptr;            // the engine's stream (the context's unless set before init)
   cudaStream_t side = nullptr;              // captures the regeneration loop's body
-  std::map<int, cudaGraphExec_t> graphs;   // captured pass by (depth, shadow stage)
+  std::map<int, cudaGraphExec_t> graphs;   // captured pass by (depth, path kernel alone, shadow stage)
   std::map<int, cudaGraphExec_t> head_graphs;   // the same without accumulate and advance
   cudaGraphExec_t acc_graph = nullptr;          // accumulate + advance
   long long passes = 0, launches = 0;
@@ -74,7 +75,13 @@ struct Engine {
   int read_row_rays(int r, unsigned long long* out);   // synchronous
   int free_rows() const;
   long long paths_in_pass() const;                      // of the next pass, from the mirror
-  static int launches_per_pass(int depth, bool nee = false) { return 5 + (nee ? 3 : 2) * depth; }
+  // Launches of the next pass with `depth` bounces.
+  int launches_per_pass(int depth, bool nee = false) const {
+    if (path_pass(depth)) return 5;
+    int n = 5 + (nee ? 3 : 2) * depth;
+    for (int b = 2; b < depth; ++b) n += hand_over(b);
+    return n;
+  }
   // Launches of regenerating passes with `iterations` loop iterations in all.
   static long long launches_regen(long long passes, long long iterations, bool nee = false) {
     return 5 * passes + (nee ? 5 : 4) * iterations;
@@ -86,6 +93,17 @@ struct Engine {
   int alloc_paths(std::string* err);
   void point();
   void advance_mirror();
+  // Whether the next pass is small enough to run as one path-kernel launch. (With depth 0
+  // nothing is traced and the camera-ray stage alone clears the radiance.)
+  bool path_pass(int depth) const {
+    return paths_kernel_for(knobs) && !regen && depth > 0 && paths_in_pass() <= kPathPass;
+  }
+  // Whether a larger pass offers the rays queued for bounce b to the path kernel. A launch
+  // that declines costs about 2 us: at every bounce up to 4 and then at 6, 8, 12, 16, ...
+  // the Cornell box (256x256, 64 samples) lost 1.5%, at the powers of two from 2 nothing,
+  // and the other scenes were within 2% of either.
+  bool hand_over(int b) const { return paths_kernel_for(knobs) && !regen && b >= 2 && (b & (b - 1)) == 0; }
+  int graph_key(int depth, bool nee) const { return 4 * depth + (path_pass(depth) ? 2 : 0) + (nee ? 1 : 0); }
   int launch_head(cudaStream_t st, int depth, bool nee);
   int launch_pass(cudaStream_t st, int depth, bool nee);
   void launch_iteration(cudaStream_t st, cudaGraphConditionalHandle cond, bool use_cond, int depth, bool nee);

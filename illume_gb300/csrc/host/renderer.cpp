@@ -211,6 +211,8 @@ int Renderer::render_device(bool accumulate, illume_render_stats* stats) {
                                     cudaMemcpyDeviceToHost, st));
   }
   const int npasses = spp > 0 ? (spp + per_pass - 1) / per_pass : 0;
+  std::vector<long long> launches_before(nengines);
+  for (int e = 0; e < nengines; ++e) launches_before[e] = engine(e).launches;
   ILLUME_CUDA_TRY(cudaEventRecord(ev0, st));
   if (nengines > 1) {
     // passes go round the engines; each accumulation waits for the previous one
@@ -267,8 +269,9 @@ int Renderer::render_device(bool accumulate, illume_render_stats* stats) {
     stats->paths = (int64_t)spp * npix;
     stats->render_ms = ms;
     const bool nee = p.estimator == ILLUME_ESTIMATOR_NEE;
-    stats->kernel_launches = eng.regen ? Engine::launches_regen(npasses, iters, nee)
-                                       : (int64_t)npasses * Engine::launches_per_pass(p.max_depth, nee);
+    int64_t launched = 0;
+    for (int e = 0; e < nengines; ++e) launched += engine(e).launches - launches_before[e];
+    stats->kernel_launches = eng.regen ? Engine::launches_regen(npasses, iters, nee) : launched;
     stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wall0).count();
     stats->h2d_bytes = 4 * sizeof(int);
     stats->d2h_bytes = 16 + 3 * sizeof(int) * (size_t)nengines;

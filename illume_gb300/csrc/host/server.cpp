@@ -553,7 +553,7 @@ int Server::step(int* running_out) {
     if (depth == 0 && e.paths_in_pass() == 0) continue;
     k = std::max(k, 1);
     // (under regeneration the launches are counted when the passes are done)
-    const int per_pass_launches = e.regen ? 0 : Engine::launches_per_pass(depth, e.any_nee());
+    const int per_pass_launches = e.regen ? 0 : e.launches_per_pass(depth, e.any_nee());
     ILLUME_CUDA_TRY(cudaStreamWaitEvent(e.stream, ev0, 0));   // after admission's clears
     if ((st = e.run(k, depth)) != ILLUME_OK) return st;
     ILLUME_CUDA_TRY(cudaEventRecord(se.lane->done, e.stream));

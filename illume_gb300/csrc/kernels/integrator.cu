@@ -10,30 +10,9 @@
 // depends only on its own job row (scene, camera, Philox key, sample index), never on
 // which other jobs share the pass.
 #include "launch.h"
-#include "nee.cuh"
-#include "shading.cuh"
-#include "../common/philox.cuh"
+#include "stages.cuh"
 
 namespace illume {
-
-__device__ __forceinline__ int* ev_counts2(const WaveBuffers& w, int parity) { return w.counters + 2 + 16 * parity; }
-
-// Row of the job table that owns index x of a pass-wide numbering (paths or pixels):
-// the last row whose first index is <= x. Rows with nothing in the pass share their
-// first index with the next row, so the search passes over them.
-__device__ __forceinline__ int find_row(const int* base, int n, int x) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(base + mid) <= x) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo - 1;
-}
-
-__device__ __forceinline__ float pack_job_medium(int job, int medium) {
-  return __int_as_float((job << kMediumBits) | (medium + 1));
-}
 
 // Prefix sums of the pass's paths and pixels over the job table (one block). A table
 // whose paths would exceed the slot capacity runs no pass and raises counters[42].
@@ -103,67 +82,19 @@ __global__ void __launch_bounds__(1024) k_plan(WaveBuffers w) {
     w.counters[48] = 0;   // shadow-ray fetch counters by bounce parity
     w.counters[49] = 0;
     if (over) w.counters[42] = 1;
-    for (int c = 0; c < EV_COUNT; ++c) ev_counts2(w, 0)[c] = 0;
+    for (int c = 0; c < EV_COUNT; ++c) ev_counts(w, 0)[c] = 0;
   }
 }
 
-// init_rays, src/renderer.cu:81-110, for path slot g of job row j: pid = g - path_base
-// = sample_in_pass * npix + pixel.
-// Pixel of queue position q (0 <= q < w * h) when a sample's camera rays are queued in
-// 8x4 tiles: the pixels of whole tiles first, tile after tile in row-major order (so a
-// warp's 32 rays cover a compact patch of the image and traverse alike), then the pixels
-// of the partial tiles at the right and bottom edges in row-major order.
-__device__ __forceinline__ int tiled_pixel(int q, int w, int h) {
-  const int tw = w >> 3, th = h >> 2;
-  const int full = tw * th * 32;
-  if (q < full) {
-    const int t = q >> 5, k = q & 31;
-    return ((t / tw) * 4 + (k >> 3)) * w + (t % tw) * 8 + (k & 7);
-  }
-  const int r = q - full, rw = w - tw * 8, right = th * 4 * rw;
-  if (r < right) return (r / rw) * w + tw * 8 + r % rw;
-  return th * 4 * w + (r - right);
-}
-
-// Starts path i of the pass (0 <= i < the pass's paths) at position q of queue `par`.
+// Starts path i of the pass at position q of queue `par`.
 __device__ __forceinline__ void start_path(const WaveBuffers& w, int i, int q, int par) {
-  const int j = find_row(w.job_path_base, w.njobs, i);
-  const JobDesc& J = w.jobs[j];
-  const int npix = J.npix;
-  const CameraView& cam = J.cam;
-  // path i (in tile order) is this pixel's; its slot g keys the radiance
-  // the pass's samples come in groups of k; a group's paths are queued pixel by pixel
-  // (pixels in tile order) with the group's k samples of a pixel next to each other
-  const int rel = i - J.path_base;
-  const int ns = J.nsamples > 0 ? J.nsamples : 1;
-  const int k = w.ray_group > 1 ? (w.ray_group < ns ? w.ray_group : ns) : 1;
-  const int grp = rel / (k * npix);
-  const int kk = (grp + 1) * k <= ns ? k : ns - grp * k;   // the last group may be smaller
-  const int within = rel - grp * k * npix;
-  const int s = grp * k + within % kk;
-  const int pixel = tiled_pixel(within / kk, cam.width, cam.height);
-  const int g = J.path_base + s * npix + pixel;
-  const int sample = J.sample_base + s;
-  RngStream rng;
-  rng.init((uint32_t)pixel, (uint32_t)sample, 0u, J.seed, J.job);
-  const int x = pixel % cam.width, y = pixel / cam.width;
-  const float left_edge = cam.left + cam.pixel_size * (float)x;
-  const float top_edge = cam.top - cam.pixel_size * (float)y;
-  const float r_x = left_edge + cam.pixel_size * rng.next();
-  const float r_y = top_edge - cam.pixel_size * rng.next();
-  V3 pos = v3(0.0f, 0.0f, 0.0f);
-  if (cam.aperture > FLT_EPSILON) {
-    const float u1 = rng.next(), u2 = rng.next();
-    pos = mul(sample_circle(u1, u2), cam.aperture);
-  }
-  const V3 origin = xform(cam.m, pos, 1.0f);
-  const V3 image_pos = xform(cam.m, v3(r_x, r_y, cam.dof), 1.0f);
-  const V3 dir = normalize(sub(image_pos, origin));
-  w.q_orig[par][q] = make_float4(origin.x, origin.y, origin.z, __int_as_float(g));
-  w.q_dir[par][q] = make_float4(dir.x, dir.y, dir.z, pack_job_medium(j, -1));
+  float4 qo, qd;
+  camera_path(w, i, qo, qd);
+  w.q_orig[par][q] = qo;
+  w.q_dir[par][q] = qd;
   w.q_thr[par][q] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
   if (w.q_bounce[par]) w.q_bounce[par][q] = 0;
-  w.contrib[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  w.contrib[__float_as_int(qo.w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
 __global__ void __launch_bounds__(256) k_raygen(WaveBuffers w) {
@@ -233,23 +164,6 @@ __global__ void k_regen_plan(WaveBuffers w, cudaGraphConditionalHandle cond, int
   if (use_cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 
-// A path's radiance: the reference estimator ends a path at its one contribution, so
-// the slot is written once; with next-event estimation contributions add up.
-template <bool NEE>
-__device__ __forceinline__ void add_radiance(float4* c, V3 L) {
-  if (NEE) {
-    const float4 v = *c;
-    *c = make_float4(v.x + L.x, v.y + L.y, v.z + L.z, 0.0f);
-  } else {
-    *c = make_float4(L.x, L.y, L.z, 0.0f);
-  }
-}
-
-struct BounceRng {
-  RngStream s;
-  __device__ __forceinline__ float operator()() { return s.next(); }
-};
-
 // Shading of one bounce over the material-sorted event queues. MINB = blocks of 128
 // threads per SM the register allocation must allow (1 = the compiler's choice).
 // NEE: the instance with the next-event estimator compiled in (launched only when a job
@@ -258,7 +172,7 @@ template <int MINB, bool NEE>
 __global__ void __launch_bounds__(128, MINB) k_shade(WaveBuffers w, int bounce_arg) {
   const int it = pass_iteration(w, bounce_arg);
   const int parity = it & 1;
-  const int* counts = ev_counts2(w, parity);
+  const int* counts = ev_counts(w, parity);
   __shared__ int prefix[EV_COUNT + 1];
   // block-level aggregation of the counters every warp would otherwise hit with its own
   // atomic (one address each, so those atomics serialise in L2): the rays of the block's
@@ -276,7 +190,7 @@ __global__ void __launch_bounds__(128, MINB) k_shade(WaveBuffers w, int bounce_a
   }
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    int* next_counts = ev_counts2(w, parity ^ 1);
+    int* next_counts = ev_counts(w, parity ^ 1);
     for (int c = 0; c < EV_COUNT; ++c) next_counts[c] = 0;
     atomicAdd(w.rays, (unsigned long long)w.counters[parity]);
   }
@@ -284,10 +198,10 @@ __global__ void __launch_bounds__(128, MINB) k_shade(WaveBuffers w, int bounce_a
   int* next_count = w.counters + (parity ^ 1);
   for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
     const int gi = base + threadIdx.x;
-    bool cont = false, shadow = false;
-    int myjob = -1;
-    float4 no = make_float4(0, 0, 0, 0), nd = no, nt = no;
-    float4 so = no, sd = no, sv = no;
+    ShadeOut out;
+    out.cont = out.shadow = false;
+    out.no = make_float4(0, 0, 0, 0);
+    out.nd = out.nt = out.so = out.sd = out.sv = out.no;
     int bounce = it;   // this ray's bounce (per ray under path regeneration)
     const unsigned live = __ballot_sync(0xffffffffu, gi < total);
     if (gi < total) {
@@ -304,171 +218,25 @@ __global__ void __launch_bounds__(128, MINB) k_shade(WaveBuffers w, int bounce_a
       const bool no_hit = cls == EV_MISS || cls == EV_MEDIUM;
       const float4 hv = no_hit ? make_float4(FLT_MAX, 0.0f, 0.0f, __int_as_float(-1)) : w.hit[i];
       const int geom = no_hit ? -1 : w.hit_geom[i];
-      const int g = __float_as_int(qo.w);
-      const int packed = __float_as_int(qd.w);
-      const int job = packed >> kMediumBits;
-      myjob = job;
-      int medium = (packed & ((1 << kMediumBits) - 1)) - 1;
-      const JobDesc& J = w.jobs[job];
-      const SceneView sc = J.sc;
-      const int pid = g - J.path_base;
-      const int npix = J.npix;
-      const V3 o = v3(qo.x, qo.y, qo.z), d = v3(qd.x, qd.y, qd.z);
-      V3 thr = v3(qt.x, qt.y, qt.z);
-      const float t = hv.x;
-      BounceRng rng;
-      rng.s.init((uint32_t)(pid % npix), (uint32_t)(J.sample_base + pid / npix), (uint32_t)(bounce + 1), J.seed,
-                 J.job);
-      float4* contrib = w.contrib + g;
-      const bool last = bounce + 1 >= J.max_depth;
-      const bool nee = NEE && (J.flags & JOB_NEE) != 0;
-      const float pdf_prev = qt.w;   // density of the BSDF sample that led here (next-event paths)
-      if (medium >= 0 && sc.mediums[medium].active) {
-        const DevMedium md = sc.mediums[medium];
-        const float u = rng();
-        const float dist = -logf(u) / md.scattering;
-        if (cls == EV_MEDIUM) {
-          const float u1 = rng(), u2 = rng();
-          const V3 dir = to_basis(sample_hg(md.g, u1, u2, (J.flags & JOB_EXACT_HG) != 0), d);
-          const V3 no3 = add(o, mul(d, dist));
-          const V3 nd3 = normalize(dir);
-          thr = mulv(thr, v3(expf(-1.0f * dist * md.absorption[0]), expf(-1.0f * dist * md.absorption[1]),
-                             expf(-1.0f * dist * md.absorption[2])));
-          if (!((double)length2(thr) < 1e-4) && !last) {
-            cont = true;
-            no = make_float4(no3.x, no3.y, no3.z, qo.w);
-            nd = make_float4(nd3.x, nd3.y, nd3.z, qd.w);
-            nt = make_float4(thr.x, thr.y, thr.z, 0.0f);
-          }
-          goto done;
-        }
-        thr = mulv(thr, v3(expf(-1.0f * t * md.absorption[0]), expf(-1.0f * t * md.absorption[1]),
-                           expf(-1.0f * t * md.absorption[2])));
-      }
-      if (cls == EV_MISS) {
-        V3 L = mulv(thr, env_eval(sc, d));
-        if (nee && pdf_prev > 0.0f) L = mul(L, power_heuristic(pdf_prev, env_light_pdf(*sc.lights, d)));
-        add_radiance<NEE>(contrib, L);
-        goto done;
-      }
-      {
-        // shading frame of the hit
-        V3 N;
-        float uv0, uv1;
-        int matid;
-        if (geom >= 0) {
-          const DevInstance& in = sc.instances[geom];
-          const DevMesh& m = sc.meshes[in.mesh];
-          const int prim = __float_as_int(hv.w);
-          const int i0 = __ldg(m.tris + 3 * prim), i1 = __ldg(m.tris + 3 * prim + 1), i2 = __ldg(m.tris + 3 * prim + 2);
-          const float bu = hv.y, bv = hv.z;
-          V3 n;
-          if (!m.normals) {
-            const V3 v0 = v3(__ldg(m.positions + 3 * i0), __ldg(m.positions + 3 * i0 + 1), __ldg(m.positions + 3 * i0 + 2));
-            const V3 v1 = v3(__ldg(m.positions + 3 * i1), __ldg(m.positions + 3 * i1 + 1), __ldg(m.positions + 3 * i1 + 2));
-            const V3 v2 = v3(__ldg(m.positions + 3 * i2), __ldg(m.positions + 3 * i2 + 1), __ldg(m.positions + 3 * i2 + 2));
-            n = normalize(cross(sub(v1, v0), sub(v2, v0)));
-          } else {
-            const V3 n0 = v3(__ldg(m.normals + 3 * i0), __ldg(m.normals + 3 * i0 + 1), __ldg(m.normals + 3 * i0 + 2));
-            const V3 n1 = v3(__ldg(m.normals + 3 * i1), __ldg(m.normals + 3 * i1 + 1), __ldg(m.normals + 3 * i1 + 2));
-            const V3 n2 = v3(__ldg(m.normals + 3 * i2), __ldg(m.normals + 3 * i2 + 1), __ldg(m.normals + 3 * i2 + 2));
-            n = normalize(add(mul(n0, 1.0f - bu - bv), add(mul(n1, bu), mul(n2, bv))));
-          }
-          N = normalize(xform(in.trans_inv, n, 0.0f));
-          if (m.texcoords) {
-            const float w0 = 1.0f - bu - bv;
-            uv0 = (__ldg(m.texcoords + 2 * i0) * w0 + __ldg(m.texcoords + 2 * i1) * bu) + __ldg(m.texcoords + 2 * i2) * bv;
-            uv1 = (__ldg(m.texcoords + 2 * i0 + 1) * w0 + __ldg(m.texcoords + 2 * i1 + 1) * bu) +
-                  __ldg(m.texcoords + 2 * i2 + 1) * bv;
-          } else {
-            uv0 = bu;
-            uv1 = bv;
-          }
-          matid = in.material;
-        } else {
-          const DevSphere sp = sc.spheres[-2 - geom];
-          const V3 pos = add(o, mul(d, t));
-          N = normalize(sub(pos, v3(sp.cx, sp.cy, sp.cz)));
-          uv0 = (float)((double)(atan2f(N.z, N.x) * 0.5f) * ILLUME_INV_PI_D + 0.5);
-          uv1 = (float)(0.5 - (double)asinf(N.y) * ILLUME_INV_PI_D);
-          matid = sp.material;
-        }
-        const DevMaterial mat = sc.materials[matid];
-        const V3 albedo = tex_eval(sc, mat.albedo_tex, uv0, uv1);
-        const float roughness = tex_eval(sc, mat.roughness_tex, uv0, uv1).x;
-        if (mat.type == MAT_EMISSIVE) {
-          V3 L = mulv(thr, albedo);
-          if (nee && pdf_prev > 0.0f && geom >= 0) {
-            const LightView& LV = *sc.lights;
-            const int base = LV.num_tri > 0 ? __ldg(LV.inst_light_base + geom) : -1;
-            if (base >= 0) {
-              const int l = base + __float_as_int(hv.w);
-              const float4 e1 = __ldg(&LV.tri[3 * l + 1]), e2 = __ldg(&LV.tri[3 * l + 2]);
-              const V3 ln = cross(v3(e1.x, e1.y, e1.z), v3(e2.x, e2.y, e2.z));
-              const float lnl = sqrtf(dot(ln, ln));
-              const float cos_l = lnl > 0.0f ? dot(ln, d) / lnl : 0.0f;
-              L = mul(L, power_heuristic(pdf_prev, tri_light_pdf(LV, l, t, cos_l)));
-            }
-          }
-          add_radiance<NEE>(contrib, L);
-          goto done;
-        }
-        if (last) goto done;   // the path has used all its closest-hit queries
-        // next-event estimation: one light sample at a non-delta reflection vertex in air
-        if (nee && (medium < 0 || !sc.mediums[medium].active) &&
-            (mat.type == MAT_LAMBERT || mat.type == MAT_ROUGHCONDUCTOR || mat.type == MAT_ROUGHREFLECTIVE)) {
-          RngStream nr;
-          nr.init((uint32_t)(pid % npix), (uint32_t)(J.sample_base + pid / npix), 0x40000000u | (uint32_t)(bounce + 1),
-                  J.seed, J.job);
-          const float u0 = nr.next(), u1 = nr.next(), u2 = nr.next();
-          const V3 ph = add(o, mul(d, t));
-          const LightSample ls = sample_light(sc, *sc.lights, ph, u0, u1, u2);
-          V3 fcos;
-          float pdf_b = 0.0f;
-          if (ls.ok && bsdf_eval_cos(mat, d, N, albedo, roughness, ls.dir, fcos, pdf_b)) {
-            const V3 Cn = mul(mulv(mulv(thr, fcos), ls.Le), power_heuristic(ls.pdf, pdf_b) / ls.pdf);
-            if (isfinite(Cn.x + Cn.y + Cn.z) && (Cn.x > 0.0f || Cn.y > 0.0f || Cn.z > 0.0f)) {
-              const V3 norm_o = mul(N, dot(N, d) > 0.0f ? -1.0f : 1.0f);
-              const V3 org = add(ph, mul(norm_o, J.ray_bias));
-              const float tmax = ls.dist == FLT_MAX ? FLT_MAX : ls.dist * (1.0f - 1e-4f) - J.ray_bias;
-              if (tmax > 0.0f) {
-                shadow = true;
-                so = make_float4(org.x, org.y, org.z, __int_as_float(job));
-                sd = make_float4(ls.dir.x, ls.dir.y, ls.dir.z, tmax);
-                sv = make_float4(Cn.x, Cn.y, Cn.z, __int_as_float(g));
-              }
-            }
-          }
-        }
-        const ScatterResult s = scatter(mat, d, N, albedo, roughness, rng);
-        if (s.status == SCATTER_KILLED) goto done;
-        if (s.medium != kMediumUnchanged) medium = s.medium;
-        thr = mulv(thr, s.weight);
-        const V3 p = add(add(o, mul(d, t)), mul(s.offset_dir, s.offset_sign * J.ray_bias));
-        const V3 dir = normalize(s.dir);
-        cont = true;
-        no = make_float4(p.x, p.y, p.z, qo.w);
-        nd = make_float4(dir.x, dir.y, dir.z, pack_job_medium(job, medium));
-        nt = make_float4(thr.x, thr.y, thr.z, nee ? bsdf_sampled_pdf(mat, s, d, N) : 0.0f);
-      }
-    done:;
+      const int job = __float_as_int(qd.w) >> kMediumBits;
       // closest-hit queries of this bounce, per job: the block's first job in shared
       // memory, any other job with a global atomic
-      const unsigned peers = __match_any_sync(live, myjob);
+      const unsigned peers = __match_any_sync(live, job);
       if (lane == __ffs(peers) - 1) {
         int bj = *(volatile int*)&s_job;
         if (bj < 0) {
-          atomicCAS(&s_job, -1, myjob);
+          atomicCAS(&s_job, -1, job);
           bj = *(volatile int*)&s_job;
         }
-        if (bj == myjob) atomicAdd(&s_rays, (unsigned long long)__popc(peers));
-        else atomicAdd(&w.jobs[myjob].rays, (unsigned long long)__popc(peers));
+        if (bj == job) atomicAdd(&s_rays, (unsigned long long)__popc(peers));
+        else atomicAdd(&w.jobs[job].rays, (unsigned long long)__popc(peers));
       }
+      shade_event<NEE>(w, w.jobs[job], cls, qo, qd, qt, hv, geom, bounce, out);
     }
     // compacted appends of the shadow rays and of the continuing paths: one atomic per
     // block and queue (the loop's trip count is uniform over the block)
-    const unsigned ballot = __ballot_sync(0xffffffffu, cont);
-    const unsigned sballot = NEE ? __ballot_sync(0xffffffffu, shadow) : 0u;
+    const unsigned ballot = __ballot_sync(0xffffffffu, out.cont);
+    const unsigned sballot = NEE ? __ballot_sync(0xffffffffu, out.shadow) : 0u;
     if (lane == 0) {
       s_warp_cnt[0][warp] = __popc(ballot);
       if (NEE) s_warp_cnt[1][warp] = __popc(sballot);
@@ -482,17 +250,17 @@ __global__ void __launch_bounds__(128, MINB) k_shade(WaveBuffers w, int bounce_a
     }
     __syncthreads();
     const unsigned below = (1u << lane) - 1;
-    if (NEE && shadow) {
+    if (NEE && out.shadow) {
       const int j = s_base[1] + s_warp_base[1][warp] + __popc(sballot & below);
-      w.s_orig[j] = so;
-      w.s_dir[j] = sd;
-      w.s_val[j] = sv;
+      w.s_orig[j] = out.so;
+      w.s_dir[j] = out.sd;
+      w.s_val[j] = out.sv;
     }
-    if (cont) {
+    if (out.cont) {
       const int j = s_base[0] + s_warp_base[0][warp] + __popc(ballot & below);
-      w.q_orig[parity ^ 1][j] = no;
-      w.q_dir[parity ^ 1][j] = nd;
-      w.q_thr[parity ^ 1][j] = nt;
+      w.q_orig[parity ^ 1][j] = out.no;
+      w.q_dir[parity ^ 1][j] = out.nd;
+      w.q_thr[parity ^ 1][j] = out.nt;
       if (w.q_bounce[parity ^ 1]) w.q_bounce[parity ^ 1][j] = bounce + 1;
     }
   }

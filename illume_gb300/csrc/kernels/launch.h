@@ -113,6 +113,7 @@ static constexpr int kCounterMore = 56;
 static constexpr int kCounterLoopLimit = 57;
 static constexpr int kCounterIterTotal = 58;
 static constexpr int kCounterPixels = 41;
+static constexpr int kCounterPathTicket = 59;   // blocks of the path kernel that are done (0 between launches)
 static constexpr int kCounterWords = 64;
 
 // Iteration of a stage launched with `bounce` (-1 under path regeneration: read from the
@@ -127,6 +128,23 @@ __device__ __forceinline__ int ray_bounce(const WaveBuffers& w, int parity, int 
 // Samples of a pixel kept together in a pass's camera-ray queue by default (traversal
 // workload, Mrays/s: 1 -> 4168, 4 -> 4249, 8 -> 4311, 16 -> 4349, 32 -> 4266).
 static constexpr int kDefaultRayGroup = 16;
+
+// The path kernel (paths.cu): blocks of 128 per SM (at most 128 registers, no spills; 5 and
+// 6 blocks spill: a 64x48 render 7-19% slower, a 1280x720 sample 5%), the largest pass that runs as one launch of it, and
+// the rays at which a larger pass hands the rest of its paths over.
+// Pass of 12 bounces, ms, wavefront with hand-over / one path-kernel launch, by paths:
+//              2^14        2^16        2^17        2^18        2^19        2^20
+//   Cornell    .21 / .12   .22 / .14   .27 / .19   .33 / .32   .48 / .56   .80 / 1.06
+//   mixed      .47 / .34   .54 / .45   .63 / .48   .74 / .57   .86 / .70  1.13 / 1.08
+//   medium     .38 / .25   .47 / .35   .60 / .52   .93 / .97  1.41 / 1.84 2.14 / 3.58
+//   NEE        .48 / .28   .64 / .45   .75 / .61   .96 / 1.01 1.20 / 1.76 1.63 / 3.24
+// The wavefront runs lanes of one event class together, which pays once a bounce fills the
+// device several times over (311,296 lanes at 64 registers). Hand-over at 2^16 / 2^17 /
+// 2^18 / 2^19 rays: textured scene 2.54 / 2.19 / 2.21 / 2.37 ms, light sampling 7.02 /
+// 7.17 / 7.18 / 7.59, 16 large meshes 5.65 / 5.63 / 5.62 / 5.89.
+static constexpr int kPathBlocks = 4;
+static constexpr int kPathPass = 1 << 18;
+static constexpr int kPathTail = 1 << 17;
 
 // Settings shared by every job of a table (they select kernel instances).
 struct RenderKnobs {
@@ -157,6 +175,12 @@ void launch_trace(const WaveBuffers& w, const RenderKnobs& k, int bounce, int gr
                   bool count_visits = false);
 void launch_shade(const WaveBuffers& w, const RenderKnobs& k, int bounce, int grid, cudaStream_t st, bool nee = false);
 void launch_shadow(const WaveBuffers& w, const RenderKnobs& k, int bounce, int grid, cudaStream_t st);
+// Path kernel (paths.cu): bounce < 0 starts every path of the pass and runs it to its end;
+// bounce >= 1 takes over the rays queued for that bounce when there are at most `limit`
+// (and leaves the queue empty). For the settings paths_kernel_for accepts.
+bool paths_kernel_for(const RenderKnobs& k);
+void launch_paths(const WaveBuffers& w, const RenderKnobs& k, int bounce, int depth, int limit, int grid,
+                  cudaStream_t st, bool nee = false);
 void launch_accumulate(const WaveBuffers& w, int grid, cudaStream_t st);
 void launch_advance(const WaveBuffers& w, cudaStream_t st);
 void launch_tonemap(const Accumulators& acc, int accum_mode, int npix, float samples, int op, uint8_t* rgb8,
@@ -175,5 +199,6 @@ void launch_l2_read(const void* buf, size_t bytes, int reps, unsigned* sink, int
 const void* l2_read_kernel_ptr();
 const void* shade_kernel_ptr(int variant = 0, bool nee = false);
 const void* shadow_kernel_ptr(int bvh_kind);
+const void* paths_kernel_ptr(int isect, bool nee);
 
 }  // namespace illume

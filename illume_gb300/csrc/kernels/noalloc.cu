@@ -114,7 +114,7 @@ extern "C" int illume_render_noalloc(illume_context* ctx, illume_scene* scene, c
   const int dev = ctx->c.device;
   ILLUME_CUDA_TRY(cudaSetDevice(dev));
   void* base = nullptr;
-  int grid_trace = 0, grid_shade = 0;
+  int grid_trace = 0, grid_shade = 0, grid_paths = 0;
   {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     void* cu_ctx = current_driver_context();
@@ -133,6 +133,9 @@ extern "C" int illume_render_noalloc(illume_context* ctx, illume_scene* scene, c
     if (!gt) gt = kernel_grid_blocks(trace_kernel_ptr(k.bvh_kind, k.trace_variant), 128, dev);
     int& gs = ctx->c.noalloc_grid_shade[k.shade_variant & 7];
     if (!gs) gs = kernel_grid_blocks(shade_kernel_ptr(k.shade_variant), 128, dev);
+    int& gp = ctx->c.noalloc_grid_paths[k.isect & 1];
+    if (!gp) gp = kernel_grid_blocks(paths_kernel_ptr(k.isect, false), 128, dev);
+    grid_paths = gp;
     grid_trace = gt;
     grid_shade = gs;
   }
@@ -172,17 +175,24 @@ extern "C" int illume_render_noalloc(illume_context* ctx, illume_scene* scene, c
   const int sms = ctx->c.sm_count > 0 ? ctx->c.sm_count : 1;
   const int grid_small = std::max(1, std::min((cap + 255) / 256, sms * 8));
   k_noalloc_begin<<<grid_small, 256, 0, st>>>(w.counters, w.rays, w.visits, w.jobs, row, d_sum, cap);
+  // a pass of at most kNoAllocMaxPaths paths is within the path kernel's range
+  static_assert(kNoAllocMaxPaths <= (size_t)kPathPass, "passes of this entry point run as one path-kernel launch");
+  const bool paths = paths_kernel_for(k) && p.max_depth > 0;
   for (int s = 0; s < p.spp; ++s) {
     launch_plan(w, st);
-    launch_raygen(w, grid_small, st);
-    for (int b = 0; b < p.max_depth; ++b) {
-      launch_trace(w, k, b, grid_trace, st);
-      launch_shade(w, k, b, grid_shade, st);
+    if (paths) {
+      launch_paths(w, k, -1, p.max_depth, 0, grid_paths, st);
+    } else {
+      launch_raygen(w, grid_small, st);
+      for (int b = 0; b < p.max_depth; ++b) {
+        launch_trace(w, k, b, grid_trace, st);
+        launch_shade(w, k, b, grid_shade, st);
+      }
     }
     launch_accumulate(w, grid_small, st);
     launch_advance(w, st);
   }
   ILLUME_CUDA_TRY(cudaGetLastError());
-  ctx->c.launches += 1 + (long long)p.spp * (4 + 2 * p.max_depth);
+  ctx->c.launches += 1 + (long long)p.spp * (paths ? 4 : 4 + 2 * p.max_depth);
   return ILLUME_OK;
 }

@@ -2,13 +2,11 @@
 #include <type_traits>
 
 #include "launch.h"
+#include "stages.cuh"
 #include "trace.cuh"
-#include "../common/philox.cuh"
 #include "../../../include/illume.h"
 
 namespace illume {
-
-__device__ __forceinline__ int* ev_counts(const WaveBuffers& w, int parity) { return w.counters + 2 + 16 * parity; }
 
 // Warp-aggregated append: lanes of `mask` that pass the same `key` share one atomic.
 __device__ __forceinline__ int warp_append_keyed(unsigned mask, int key, int* counters) {
@@ -21,42 +19,12 @@ __device__ __forceinline__ int warp_append_keyed(unsigned mask, int key, int* co
   return base + __popc(peers & ((1u << lane) - 1));
 }
 
-// Distance at which a ray in an active medium scatters: the first number of the path's
-// bounce stream, as src/renderer.cu:152-157 draws it.
-__device__ __forceinline__ float medium_distance(const JobDesc& J, const SceneView& sc, int g, int medium, int bounce) {
-  const int pid = g - J.path_base;
-  const uint32_t pixel = (uint32_t)(pid % J.npix), sample = (uint32_t)(J.sample_base + pid / J.npix);
-  const Philox4 r = philox4x32_10(pixel, sample, (uint32_t)(bounce + 1), 0u, J.seed, J.job);
-  return -logf(philox_unit(r.x)) / sc.mediums[medium].scattering;
-}
-
-__device__ __forceinline__ int surface_class(const SceneView& sc, const HitRecord& h) {
-  if (h.geom == -1) return EV_MISS;
-  const int mat = h.geom >= 0 ? sc.instances[h.geom].material : sc.spheres[-2 - h.geom].material;
-  return EV_SURFACE + sc.materials[mat].type;
-}
-
 // Event class of a traced ray: escape, medium scatter before the surface, or the hit
 // material.
 __device__ __forceinline__ int event_class(const WaveBuffers& w, const JobDesc& J, const SceneView& sc,
                                            const HitRecord& h, int g, int medium, int bounce) {
   if (medium >= 0 && sc.mediums[medium].active && medium_distance(J, sc, g, medium, bounce) < h.t) return EV_MEDIUM;
   return surface_class(sc, h);
-}
-
-// Search bound of a ray in an active medium. The ray scatters at `dist` unless a surface
-// lies at t <= dist, so the search need not look further: hits closer than the next float
-// above dist are the ones with t <= dist. A bounded search that finds nothing leaves its
-// bound in the hit record (never FLT_MAX), and the ray scatters; one that finds something
-// has found the surface before it. Where dist is infinite or NaN the ray cannot scatter
-// and the search has no bound (FLT_MAX).
-// Subsurface walk (200k triangles, unit mean free path in a body 120 across): 15.1 -> 6.0
-// node visits per ray, a 480x360 render at 16 samples 28.3 -> 13.8 ms.
-__device__ __forceinline__ float medium_bound(float dist) {
-  if (!(fabsf(dist) < FLT_MAX)) return dist < 0.0f ? dist : FLT_MAX;
-  const int b = __float_as_int(dist);
-  const int next = dist == 0.0f ? 1 : b + (dist > 0.0f ? 1 : -1);
-  return fminf(__int_as_float(next), 3.4028233e38f);   // the float below FLT_MAX
 }
 
 // Trace stage of one bounce: closest hit of every queued ray in its job's scene, then
@@ -82,6 +50,9 @@ __global__ void __launch_bounds__(128, MINB) k_trace(WaveBuffers w, RenderKnobs 
   typename std::conditional<KIND == BVH_WIDE8, uint2, int>::type stack[kStack];
   unsigned long long my_nodes = 0, my_tris = 0, my_slots = 0;
   int base = OPT ? 0 : blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+  // as many warps as the rays can occupy: on few rays the others' atomics on the one
+  // counter would cost more than the rays (2 us a launch for a full grid)
+  if (OPT && (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >= n) return;
   for (;;) {
     if (OPT) {
       int b0 = 0;
@@ -281,6 +252,7 @@ __global__ void __launch_bounds__(128, 8) k_shadow(WaveBuffers w, RenderKnobs k,
   int* fetch = w.counters + 48 + parity;
   const int lane = threadIdx.x & 31;
   typename std::conditional<KIND == BVH_WIDE8, uint2, int>::type stack[kStack];
+  if ((int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >= n) return;   // as in k_trace
   for (;;) {
     int b0 = 0;
     if (lane == 0) b0 = atomicAdd(fetch, 32);
