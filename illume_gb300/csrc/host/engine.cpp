@@ -75,6 +75,11 @@ static int capture_while(cudaStream_t st, cudaStream_t side, const std::function
 }
 
 int Engine::ensure_shadow(std::string* err) {
+  if (!grid_shadow) {   // the next-event kernels' grids, looked up by the tables that use them
+    grid_shadow = kernel_grid_blocks(shadow_kernel_ptr(knobs.bvh_kind), 128, ctx->device);
+    grid_shade_nee = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant, true), 128, ctx->device);
+    grid_paths_nee = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, true), 128, ctx->device);
+  }
   if (s_orig.get() && s_orig.size() >= sizeof(float4) * (size_t)qcap) return ILLUME_OK;
   int st;
   if ((st = s_orig.alloc(ctx, sizeof(float4) * (size_t)qcap)) != ILLUME_OK) { *err = last_error(); return st; }
@@ -171,10 +176,7 @@ int Engine::init(Context* c, int nrows, int ncap, const RenderKnobs& k, std::str
   point();
   grid_trace = kernel_grid_blocks(trace_kernel_ptr(knobs.bvh_kind, knobs.trace_variant), 128, ctx->device);
   grid_shade = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant), 128, ctx->device);
-  grid_shadow = kernel_grid_blocks(shadow_kernel_ptr(knobs.bvh_kind), 128, ctx->device);
-  grid_shade_nee = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant, true), 128, ctx->device);
-  grid_paths = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, false), 128, ctx->device);
-  grid_paths_nee = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, true), 128, ctx->device);
+  if (paths_kernel_for(knobs)) grid_paths = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, false), 128, ctx->device);
   return ILLUME_OK;
 }
 
@@ -221,6 +223,8 @@ int Engine::set_trace_variant(int variant) {
   drop_graphs();
   knobs.trace_variant = variant;
   grid_trace = kernel_grid_blocks(trace_kernel_ptr(knobs.bvh_kind, knobs.trace_variant), 128, ctx->device);
+  if (paths_kernel_for(knobs) && !grid_paths)
+    grid_paths = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, false), 128, ctx->device);
   return ILLUME_OK;
 }
 

@@ -339,11 +339,17 @@ __device__ __forceinline__ void sort_pair(float& ka, int& ea, float& kb, int& eb
 // arithmetic is the same, so are the results.
 // PS: four compare-swaps instead of five: the nearest child is exact, the middle two of
 // the pushed ones may come out of order (order changes the work, never the result).
-template <bool COUNT, bool ANY = false, bool PS = false, bool NF = false>
+// SB: an empty entry below the stack ends the walk when it is popped, instead of a test for
+// an empty stack at every pop, and the rare full stack is tested in front of the pushes. In
+// the general kernel the watertight scenes trace 4-8% faster with it (16 large meshes 3.62
+// -> 3.32 ms per pass, textured 2.03 -> 1.92, subsurface 10.87 -> 10.49); in the instance
+// for the Moller-Trumbore test the traversal scene loses 1% (6.55 -> 6.62).
+template <bool COUNT, bool ANY = false, bool PS = false, bool NF = false, bool SB = false>
 __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRay& r, int isect, MeshBest& best,
                                                  int* stack, VisitCount& vc) {
   constexpr int kEmpty = kEmptyEntry;
   int sp = 0, cur = 0, leaf = kEmpty, visits = 0;
+  if (SB) stack[sp++] = kEmpty;
   // near-plane offsets in a Bvh4Node: lox/loy/loz at 0/16/32, hix/hiy/hiz at 48/64/80
   const unsigned near_x = r.idir.x >= 0.0f ? 0u : 48u, near_y = r.idir.y >= 0.0f ? 16u : 64u,
                  near_z = r.idir.z >= 0.0f ? 32u : 80u;
@@ -351,7 +357,10 @@ __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRa
     if (sp < kStack) stack[sp++] = v;
     else vc.dropped = true;
   };
-  auto pop = [&]() -> int { return stack[--sp]; };
+  auto pop = [&]() -> int {
+    if (SB) return stack[--sp];
+    return sp > 0 ? stack[--sp] : kEmpty;
+  };
   do {
     while (cur >= 0) {
       if (COUNT) vc.nodes++;
@@ -386,7 +395,15 @@ __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRa
       }
       // (occlusion: any hit ends the walk, so the children go unordered.) The room for
       // the three pushes is checked once per node; a full stack drops what does not fit.
-      if (__builtin_expect(sp <= kStack - 3, 1)) {
+      if (SB) {
+        if (__builtin_expect(sp > kStack - 3, 0)) {
+          vc.dropped = true;
+          sp = kStack - 3;
+        }
+        if (e3 != kEmpty) stack[sp++] = e3;
+        if (e2 != kEmpty) stack[sp++] = e2;
+        if (e1 != kEmpty) stack[sp++] = e1;
+      } else if (__builtin_expect(sp <= kStack - 3, 1)) {
         if (e3 != kEmpty) stack[sp++] = e3;
         if (e2 != kEmpty) stack[sp++] = e2;
         if (e1 != kEmpty) stack[sp++] = e1;
@@ -395,10 +412,10 @@ __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRa
         if (e2 != kEmpty) push(e2);
         if (e1 != kEmpty) push(e1);
       }
-      cur = e0 != kEmpty ? e0 : (sp > 0 ? pop() : kEmpty);
+      cur = e0 != kEmpty ? e0 : pop();
       if (cur < kEmpty && leaf == kEmpty) {
         leaf = cur;
-        cur = sp > 0 ? pop() : kEmpty;
+        cur = pop();
       }
       if (__all_sync(__activemask(), leaf != kEmpty)) break;
     }
@@ -411,7 +428,7 @@ __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRa
       leaf = kEmpty;
       if (cur < kEmpty) {
         leaf = cur;
-        cur = sp > 0 ? pop() : kEmpty;
+        cur = pop();
       }
     }
   } while (cur != kEmpty);
@@ -721,7 +738,7 @@ __device__ __forceinline__ HitRecord closest_hit(const SceneView& sc, V3 o, V3 d
     MeshBest b{h.t, seed, 0.0f, 0.0f};
     const DevMesh& m = sc.meshes[mesh];
     if (KIND == BVH_WIDE8) traverse_wide<COUNT>(m, r, isect, b, reinterpret_cast<uint2*>(stack_mem), vc);
-    else if (KIND == BVH_WIDE4) traverse_bvh4_ww<COUNT, ANY, PS, NF>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
+    else if (KIND == BVH_WIDE4) traverse_bvh4_ww<COUNT, ANY, PS, NF, ISECT != ISECT_MT>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     else if (WW) traverse_bvh2_ww<COUNT, FMA, ANY>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     else traverse_bvh2<COUNT, FMA>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     if (b.prim >= 0 && b.prim != INT_MAX) { h.t = b.t; h.u = b.u; h.v = b.v; h.prim = b.prim; h.geom = i; }
