@@ -334,8 +334,8 @@ int illume_renderer_profile(illume_renderer* r, int count_visits, illume_profile
  * and frame loops that must not stall on cudaMalloc/cudaFree. The wavefront queues live
  * in a fixed array inside the library (about 12 MB, reserved on every GPU that loads the
  * library until exit), which limits images to ILLUME_NOALLOC_MAX_PIXELS pixels; larger
- * images are rejected with ILLUME_ERR_INVALID. Renders params->spp samples (one per
- * pass, FP32 accumulation in sample order, accum_mode must be ILLUME_ACCUM_FP32) and
+ * images are rejected with ILLUME_ERR_INVALID. Renders params->spp samples (FP32
+ * accumulation in sample order, accum_mode must be ILLUME_ACCUM_FP32) and
  * writes the per-pixel sum of radiance (3 floats per pixel) to the caller's device
  * buffer d_sum. Asynchronous on the context's stream. Takes the parameter checks of
  * illume_renderer_create; samples_per_pass and engines above 1, queue_slots above 0 and
