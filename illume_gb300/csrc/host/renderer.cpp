@@ -136,7 +136,9 @@ int Renderer::init(std::string* err) {
   acc.sum64 = sum64.as<double>();
   acc.sumsq = sumsq.as<double>();
   eng.ray_group = p.ray_group > 0 ? p.ray_group : kDefaultRayGroup;
-  if ((st = eng.init(ctx, 1, per_pass * npix, render_knobs(p), err, p.queue_slots, p.regen_threshold)) != ILLUME_OK)
+  RenderKnobs knobs = render_knobs(p);
+  knobs.overlap = nengines > 1;
+  if ((st = eng.init(ctx, 1, per_pass * npix, knobs, err, p.queue_slots, p.regen_threshold)) != ILLUME_OK)
     return st;
   JobDesc row = job_row(*scene, p, acc);
   if (nengines > 1) row.flags |= nengines << kInterleaveShift;
@@ -157,7 +159,7 @@ int Renderer::init(std::string* err) {
       Engine& x = *more.back();
       x.stream = s;
       x.ray_group = eng.ray_group;
-      if ((st = x.init(ctx, 1, per_pass * npix, render_knobs(p), err, p.queue_slots, p.regen_threshold)) != ILLUME_OK)
+      if ((st = x.init(ctx, 1, per_pass * npix, knobs, err, p.queue_slots, p.regen_threshold)) != ILLUME_OK)
         return st;
       x.mirror[0] = row;
       if ((st = x.write_row(0)) != ILLUME_OK) { *err = last_error(); return st; }

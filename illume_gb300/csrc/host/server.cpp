@@ -48,6 +48,7 @@ int Server::new_engine(const illume_render_params& p, int key, long long cap, Se
   RenderKnobs k = render_knobs(p);
   k.trace_variant = trace_variant >= 0 ? trace_variant : (p.bvh_kind == 2 ? 1 : 0);
   k.shade_variant = 0;
+  k.overlap = lanes > 1;
   std::string err;
   const int st = se.eng->init(ctx, rows, (int)cap, k, &err, queue_slots, regen_threshold);
   if (st != ILLUME_OK) { set_error(err); return st; }

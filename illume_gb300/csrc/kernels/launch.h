@@ -152,6 +152,7 @@ struct RenderKnobs {
   int bvh_kind;        // BVH_BINARY or BVH_WIDE8
   int trace_variant;   // see trace_kernel_ptr
   int shade_variant;   // see shade_kernel_ptr
+  int overlap;         // 1: passes of other tables run beside this table's (launch_trace)
 };
 
 int kernel_grid_blocks(const void* fn, int block, int device);

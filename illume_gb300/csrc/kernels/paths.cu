@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int b
       if (medium >= 0 && sc.mediums[medium].active)
         tmax = medium_bound(medium_distance(J, sc, __float_as_int(qo.w), medium, b));
       VisitCount vc;
-      const HitRecord h = closest_hit<BVH_WIDE4, false, true, false, false, false, true, true, true, ISECT>(
+      const HitRecord h = closest_hit<BVH_WIDE4, false, true, false, false, false, true, true, true>(
           sc, v3(qo.x, qo.y, qo.z), v3(qd.x, qd.y, qd.z), ISECT, stack, &vc, tmax);
       dropped |= vc.dropped;
       const int cls = h.geom == -1 && h.t != FLT_MAX ? EV_MEDIUM : surface_class(sc, h);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int b
       ++all_rays;
       if (NEE && out.shadow) {
         VisitCount sv;
-        const HitRecord s = closest_hit<BVH_WIDE4, false, false, false, true, false, true, true, false, ISECT>(
+        const HitRecord s = closest_hit<BVH_WIDE4, false, false, false, true, false, true, true, false>(
             sc, v3(out.so.x, out.so.y, out.so.z), v3(out.sd.x, out.sd.y, out.sd.z), ISECT, stack, &sv, out.sd.w);
         dropped |= sv.dropped;
         if (s.geom == -1) {

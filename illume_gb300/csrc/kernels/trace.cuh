@@ -342,8 +342,8 @@ __device__ __forceinline__ void sort_pair(float& ka, int& ea, float& kb, int& eb
 // SB: an empty entry below the stack ends the walk when it is popped, instead of a test for
 // an empty stack at every pop, and the rare full stack is tested in front of the pushes. In
 // the general kernel the watertight scenes trace 4-8% faster with it (16 large meshes 3.62
-// -> 3.32 ms per pass, textured 2.03 -> 1.92, subsurface 10.87 -> 10.49); in the instance
-// for the Moller-Trumbore test the traversal scene loses 1% (6.55 -> 6.62).
+// -> 3.32 ms per pass, textured 2.03 -> 1.92, subsurface 10.87 -> 10.49); the instances for
+// one triangle test lose up to 1% (traversal scene 6.55 -> 6.62).
 template <bool COUNT, bool ANY = false, bool PS = false, bool NF = false, bool SB = false>
 __device__ __forceinline__ void traverse_bvh4_ww(const DevMesh& m, const TraceRay& r, int isect, MeshBest& best,
                                                  int* stack, VisitCount& vc) {
@@ -738,7 +738,7 @@ __device__ __forceinline__ HitRecord closest_hit(const SceneView& sc, V3 o, V3 d
     MeshBest b{h.t, seed, 0.0f, 0.0f};
     const DevMesh& m = sc.meshes[mesh];
     if (KIND == BVH_WIDE8) traverse_wide<COUNT>(m, r, isect, b, reinterpret_cast<uint2*>(stack_mem), vc);
-    else if (KIND == BVH_WIDE4) traverse_bvh4_ww<COUNT, ANY, PS, NF, ISECT != ISECT_MT>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
+    else if (KIND == BVH_WIDE4) traverse_bvh4_ww<COUNT, ANY, PS, NF, (ISECT < 0)>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     else if (WW) traverse_bvh2_ww<COUNT, FMA, ANY>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     else traverse_bvh2<COUNT, FMA>(m, r, isect, b, reinterpret_cast<int*>(stack_mem), vc);
     if (b.prim >= 0 && b.prim != INT_MAX) { h.t = b.t; h.u = b.u; h.v = b.v; h.prim = b.prim; h.geom = i; }

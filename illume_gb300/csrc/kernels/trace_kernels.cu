@@ -476,12 +476,18 @@ __global__ void __launch_bounds__(64, KIND == BVH_WIDE4 ? (FEW ? 10 : 16) : 1)
 //   loaded by per-ray byte offsets, traversal stack in local memory (the default); 1 =
 //   four compare-swaps instead of five in the child ordering; 2 = lo and hi planes
 //   loaded and selected per child box; 3 = 6 blocks per SM (at most 80 registers).
-// The default 4-wide kernel is compiled once for the Moller-Trumbore test alone: without
-// the watertight test's six shear registers it spills nothing (132 / 368 bytes of spill
-// stores / loads otherwise). Traversal scene, 1024x1024, one 32-sample pass: 6.67 -> 6.51
-// ms of trace; Cornell box 256x256 at 64 samples: 0.61 -> 0.55 ms per pass. An instance
-// for the watertight test alone still spills 100 bytes and was 1.5% slower on 16 meshes
-// of 125k triangles (5.93 -> 6.01 ms), so that test stays in the general kernel.
+// The default 4-wide kernel has three instances, all with the same results.
+//   Moller-Trumbore test alone: without the watertight test's six shear registers it spills
+//     nothing (132 / 384 bytes of spill stores / loads otherwise). Traversal scene,
+//     1024x1024, one 32-sample pass: 6.67 -> 6.51 ms of trace; Cornell box 256x256 at 64
+//     samples: 0.61 -> 0.55 ms per pass.
+//   Watertight test alone, where passes of several tables overlap (a renderer's engines, a
+//     server's tables) and the device is full: 96 / 96 bytes of spills and fewer
+//     instructions. Renders of 17-37M paths: Cornell box 8.52 -> 8.09 ms, textured 18.05 ->
+//     17.48, instances 6.94 -> 6.79, traversal scene 8.14 -> 8.04, subsurface 38.2 -> 37.5.
+//   Either test, where a pass runs alone: a pass's last bounces are a few long searches,
+//     and the general kernel, whose test is chosen per call, finishes those sooner
+//     (subsurface 12.4 -> 12.1 ms, textured 2.10 -> 2.08, which run on one engine).
 const void* trace_kernel_ptr(int bvh_kind, int variant) {
   if (bvh_kind == BVH_WIDE4) {
     if (variant == 1) return (const void*)k_trace<BVH_WIDE4, false, 8, true, false, true, true>;
@@ -520,6 +526,8 @@ void launch_trace(const WaveBuffers& w, const RenderKnobs& k, int bounce, int gr
       if (count_visits) k_trace<BVH_WIDE4, true, 8, true, false, false, true, true, true><<<grid, 128, 0, st>>>(w, k, bounce);
       else if (k.isect == ISECT_MT)
         k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true, ISECT_MT><<<grid, 128, 0, st>>>(w, k, bounce);
+      else if (k.overlap)
+        k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true, ISECT_WATERTIGHT><<<grid, 128, 0, st>>>(w, k, bounce);
       else
         k_trace<BVH_WIDE4, false, 8, true, false, false, true, true, true><<<grid, 128, 0, st>>>(w, k, bounce);
     }

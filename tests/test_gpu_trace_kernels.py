@@ -48,3 +48,19 @@ def test_images_equal_the_binary_layouts(instances, estimator, isect):
         b, nb = image(C.BVH_BINARY, w, h, spp)
         assert na == nb and np.array_equal(a, b, equal_nan=True)
     ctx.close()
+
+
+@pytest.mark.parametrize("instances", [1, 5, 17])
+def test_overlapping_engines_give_one_engines_image(instances):
+    # the watertight test has a kernel of its own where a pass's tables overlap
+    ctx = Context(0)
+    scene = HostScene.from_data(ctx, scene_of(instances))
+    out = []
+    for engines in (1, 2, 3):
+        r = Renderer(ctx, scene, spp=7, max_depth=9, width=290, height=170, accum_mode=C.ACCUM_FP64, engines=engines)
+        o = r.render(sums=True)
+        out.append((o["sum"], o["stats"].rays))
+        r.close()
+    for s, n in out[1:]:
+        assert n == out[0][1] and np.array_equal(s, out[0][0], equal_nan=True)
+    ctx.close()
