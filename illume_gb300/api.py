@@ -190,10 +190,10 @@ class Renderer:
         """Full render; returns dict with the requested host arrays and the stats."""
         n = self.get_width() * self.get_height()
         out = {}
-        m = np.zeros((n, 3), np.float32) if mean else None
-        s = np.zeros((n, 3), np.float64) if sums else None
-        s2 = np.zeros((n, 3), np.float64) if sums else None
-        r8 = np.zeros((n, 3), np.uint8) if rgb8 else None
+        m = np.empty((n, 3), np.float32) if mean else None
+        s = np.empty((n, 3), np.float64) if sums else None
+        s2 = np.empty((n, 3), np.float64) if sums else None
+        r8 = np.empty((n, 3), np.uint8) if rgb8 else None
         st = C.RenderStats()
         C.check(C.lib().illume_render(self.handle, C.fptr(m), C.dptr(s), C.dptr(s2), C.u8ptr(r8), ctypes.byref(st)))
         out.update(mean=m, sum=s, sumsq=s2, rgb8=r8, stats=st)
@@ -206,10 +206,10 @@ class Renderer:
 
     def read(self, mean=True, sums=False, rgb8=False):
         n = self.get_width() * self.get_height()
-        m = np.zeros((n, 3), np.float32) if mean else None
-        s = np.zeros((n, 3), np.float64) if sums else None
-        s2 = np.zeros((n, 3), np.float64) if sums else None
-        r8 = np.zeros((n, 3), np.uint8) if rgb8 else None
+        m = np.empty((n, 3), np.float32) if mean else None
+        s = np.empty((n, 3), np.float64) if sums else None
+        s2 = np.empty((n, 3), np.float64) if sums else None
+        r8 = np.empty((n, 3), np.uint8) if rgb8 else None
         C.check(C.lib().illume_renderer_read(self.handle, C.fptr(m), C.dptr(s), C.dptr(s2), C.u8ptr(r8)))
         return dict(mean=m, sum=s, sumsq=s2, rgb8=r8)
 
@@ -270,8 +270,8 @@ class Server:
     def poll(self, job: int, rgb8: bool = False):
         """None while the job runs, else {'mean', 'rgb8'?, 'stats'}; raises if cancelled or failed."""
         n = self._npix[job]
-        mean = np.zeros((n, 3), np.float32)
-        px = np.zeros((n, 3), np.uint8) if rgb8 else None
+        mean = np.empty((n, 3), np.float32)
+        px = np.empty((n, 3), np.uint8) if rgb8 else None
         st = C.RenderStats()
         s = C.lib().illume_job_poll(self.handle, job, C.fptr(mean), C.u8ptr(px), ctypes.byref(st))
         if s == C.ERR_NOT_READY:
@@ -306,8 +306,8 @@ def render_batch(ctx: Context, scenes, params, autotune: bool = False, rgb8: boo
     """illume_render_batch: every job rendered together; returns ([mean per job], [rgb8 per job] or None,
     [RenderStats per job], ServerStats)."""
     n = len(scenes)
-    means = [np.zeros((p.width * p.height, 3), np.float32) for p in params]
-    pix = [np.zeros((p.width * p.height, 3), np.uint8) for p in params] if rgb8 else None
+    means = [np.empty((p.width * p.height, 3), np.float32) for p in params]
+    pix = [np.empty((p.width * p.height, 3), np.uint8) for p in params] if rgb8 else None
     sc = (ctypes.c_void_p * n)(*[s.handle.value for s in scenes])
     pa = (C.RenderParams * n)(*params)
     mp = (C._pf * n)(*[C.fptr(m) for m in means])

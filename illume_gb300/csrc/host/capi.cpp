@@ -308,9 +308,7 @@ int illume_render(illume_renderer* r, float* out_mean, double* out_sum, double* 
                   illume_render_stats* stats) {
   CHECK_ARG(r, "null renderer");
   auto t0 = std::chrono::steady_clock::now();
-  int st = r->r.render_device(false, stats);
-  if (st != ILLUME_OK) return st;
-  st = r->r.read(out_mean, out_sum, out_sumsq, out_rgb8);
+  const int st = r->r.render_and_read(out_mean, out_sum, out_sumsq, out_rgb8, stats);
   if (st != ILLUME_OK) return st;
   if (stats) {
     stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -411,14 +409,44 @@ int illume_trace_closest(illume_context* ctx, illume_scene* scene, const float* 
   CHECK_ARG(ctx && scene && n >= 0 && (n == 0 || (rays && hits)), "bad argument");
   if (n == 0) return ILLUME_OK;
   cudaSetDevice(ctx->c.device);
-  DevBuffer dr, dh;
+  Context& c = ctx->c;
+  const size_t ray_bytes = sizeof(float) * 8 * (size_t)n, hit_bytes = sizeof(illume_hit) * (size_t)n;
+  // rays, then hits: kept memory for small calls (making and freeing device memory costs
+  // more than the search of a few thousand rays), else allocated for this call
+  DevBuffer own;
   int st;
-  if ((st = dr.upload(&ctx->c, rays, sizeof(float) * 8 * (size_t)n)) != ILLUME_OK) return st;
-  if ((st = dh.alloc(&ctx->c, sizeof(illume_hit) * (size_t)n)) != ILLUME_OK) return st;
-  if ((st = illume_trace_closest_device(ctx, scene, dr.as<float>(), n, intersector, bvh_kind, dh.as<illume_hit>())) != ILLUME_OK)
+  void* mem = nullptr;
+  if (!c.budget && ray_bytes + hit_bytes <= Context::kQueryBytes) {
+    if (c.query_ws_bytes < ray_bytes + hit_bytes) {
+      if (c.query_ws) cudaFree(c.query_ws);
+      c.query_ws = nullptr;
+      c.query_ws_bytes = 0;
+      size_t want = size_t(1) << 20;
+      while (want < ray_bytes + hit_bytes) want *= 2;
+      if (cudaMalloc(&c.query_ws, want) == cudaSuccess) c.query_ws_bytes = want;
+      else { cudaGetLastError(); c.query_ws = nullptr; }
+    }
+    mem = c.query_ws;
+  }
+  if (!mem) {
+    if ((st = own.alloc(&c, ray_bytes + hit_bytes)) != ILLUME_OK) return st;
+    mem = own.get();
+  }
+  float* d_rays = static_cast<float*>(mem);
+  illume_hit* d_hits = reinterpret_cast<illume_hit*>(static_cast<char*>(mem) + ray_bytes);
+  // (1,003 rays 83 -> 74 us, 8,000 150 -> 134; past that the plain copies are as fast)
+  const bool staged = ray_bytes + hit_bytes <= Context::kStagingBytes / 2;
+  const void* from = rays;
+  if (staged) from = memcpy(c.staging(), rays, ray_bytes);
+  ILLUME_CUDA_TRY(cudaMemcpyAsync(d_rays, from, ray_bytes, cudaMemcpyHostToDevice, c.stream));
+  if ((st = illume_trace_closest_device(ctx, scene, d_rays, n, intersector, bvh_kind, d_hits)) != ILLUME_OK) {
+    cudaStreamSynchronize(c.stream);   // the copy above is done with its source
     return st;
-  ILLUME_CUDA_TRY(cudaMemcpyAsync(hits, dh.get(), sizeof(illume_hit) * (size_t)n, cudaMemcpyDeviceToHost, ctx->c.stream));
-  ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->c.stream));
+  }
+  void* to = staged ? (void*)(c.staging() + ray_bytes) : (void*)hits;
+  ILLUME_CUDA_TRY(cudaMemcpyAsync(to, d_hits, hit_bytes, cudaMemcpyDeviceToHost, c.stream));
+  ILLUME_CUDA_TRY(cudaStreamSynchronize(c.stream));
+  if (staged) memcpy(hits, to, hit_bytes);
   return ILLUME_OK;
 }
 

@@ -13,6 +13,7 @@
 // is the same as with one engine.
 #pragma once
 
+#include <chrono>
 #include <memory>
 #include <vector>
 
@@ -33,7 +34,7 @@ struct Renderer {
   int nengines = 1;
   std::vector<cudaEvent_t> acc_ev;   // per engine: its last pass's accumulation
   std::vector<cudaEvent_t> join_ev;  // per extra engine: the end of its work in a call
-  DevBuffer sum32, comp32, sum64, sumsq, out_mean, out_rgb8;
+  DevBuffer sum32, comp32, sum64, sumsq, out;   // out: mean (3 floats per pixel), then RGB8
   Accumulators acc{};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   long long samples_done = 0;   // samples accumulated since the last clear
@@ -42,17 +43,37 @@ struct Renderer {
   // defect flag, kCounterStackDrops): the image is complete but may lack hits
   bool stack_overflow = false;
   std::vector<int> iter_total;   // per engine: regeneration loop iterations read at the last call's end
+  std::vector<unsigned long long> rays_total;   // per engine: the row's ray total read at the last call's end
 
   ~Renderer();
   int init(std::string* err);
   // Renders p.spp samples; restarts the accumulation unless `accumulate`.
   int render_device(bool accumulate, illume_render_stats* stats);
   int read(float* mean, double* sum, double* sumsq, uint8_t* rgb8);
+  // Both in one call with one wait for the device.
+  int render_and_read(float* mean, double* sum, double* sumsq, uint8_t* rgb8, illume_render_stats* stats);
   // One pass launched kernel by kernel with events (see illume_renderer_profile).
   int profile(bool count_visits, illume_profile* out);
   size_t device_bytes() const;
 
  private:
+  // A call in flight: launched by enqueue (its status copies go to the context's staging
+  // memory), ended by finish after a wait for the context's stream. enqueue_read /
+  // finish_read do the same for the outputs; small mean / RGB8 images go through the
+  // staging memory as well (one copy, none of them into pageable memory).
+  struct Call {
+    int64_t launched = 0;
+    int npasses = 0;
+    std::chrono::steady_clock::time_point wall0;
+  };
+  struct Outputs {
+    bool staged = false;
+    std::vector<float> s32, c32;
+  };
+  int enqueue(bool accumulate, Call* call);
+  int finish(const Call& call, illume_render_stats* stats);
+  int enqueue_read(float* mean, double* sum, double* sumsq, uint8_t* rgb8, Outputs* out);
+  void finish_read(float* mean, double* sum, uint8_t* rgb8, const Outputs& out);
   void set_range(int first, int count);
   Engine& engine(int e) { return e == 0 ? eng : *more[e - 1]; }
 };

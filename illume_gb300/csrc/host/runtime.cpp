@@ -1,6 +1,7 @@
 #include "runtime.h"
 
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -14,6 +15,26 @@ namespace illume {
 static thread_local std::string g_error;
 void set_error(const std::string& msg) { g_error = msg; }
 const char* last_error() { return g_error.c_str(); }
+
+unsigned char* Context::staging() {
+  if (!staging_) {
+    void* q = nullptr;
+    if (cudaHostAlloc(&q, kStagingBytes, cudaHostAllocDefault) == cudaSuccess) {
+      staging_pinned_ = true;
+    } else {
+      cudaGetLastError();
+      q = malloc(kStagingBytes);
+    }
+    staging_ = static_cast<unsigned char*>(q);
+  }
+  return staging_;
+}
+
+Context::~Context() {
+  if (staging_ && staging_pinned_) cudaFreeHost(staging_);
+  else free(staging_);
+  if (query_ws) cudaFree(query_ws);
+}
 
 int DevBuffer::alloc(Context* ctx, size_t bytes) {
   release();

@@ -48,6 +48,24 @@ struct Context {
   int noalloc_grid_trace[4][8] = {};
   int noalloc_grid_shade[8] = {};
   int noalloc_grid_paths[2] = {};
+  // Page-locked host memory for the small copies of one call at a time (a context serves
+  // one thread at a time, and a call that uses it ends with a wait): made on first use,
+  // ordinary memory if the system has none to lock, freed with the context.
+  static constexpr size_t kStagingBytes = size_t(1) << 20;
+  unsigned char* staging();
+  // Device memory kept between the host-buffer query calls (at most kQueryBytes; not under
+  // a budget, which is the caller's to spend).
+  static constexpr size_t kQueryBytes = size_t(64) << 20;
+  void* query_ws = nullptr;
+  size_t query_ws_bytes = 0;
+  Context() = default;
+  Context(const Context&) = delete;
+  Context& operator=(const Context&) = delete;
+  ~Context();
+
+ private:
+  unsigned char* staging_ = nullptr;
+  bool staging_pinned_ = false;
 };
 
 // Device allocation charged against the context's budget.

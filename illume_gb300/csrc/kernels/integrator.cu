@@ -320,10 +320,11 @@ __global__ void __launch_bounds__(256) k_accumulate(WaveBuffers w) {
 }
 
 // Moves every job row to its next sample range.
-__global__ void k_advance(JobDesc* jobs, int njobs) {
+__global__ void k_advance(WaveBuffers w) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  JobDesc& J = jobs[j];
+  if (j >= w.njobs) return;
+  JobDesc& J = w.jobs[j];
+  if (j == 0) *reinterpret_cast<unsigned long long*>(w.counters + kCounterRowRays) = J.rays;
   if (J.nsamples <= 0) return;
   advance_pass_state(J.sample_base, J.nsamples, J.sample_end, J.per_pass, J.flags);
 }
@@ -464,7 +465,7 @@ void launch_shade(const WaveBuffers& w, const RenderKnobs& k, int bounce, int gr
 }
 void launch_accumulate(const WaveBuffers& w, int grid, cudaStream_t st) { k_accumulate<<<grid, 256, 0, st>>>(w); }
 void launch_advance(const WaveBuffers& w, cudaStream_t st) {
-  k_advance<<<(w.njobs + 255) / 256, 256, 0, st>>>(w.jobs, w.njobs);
+  k_advance<<<(w.njobs + 255) / 256, 256, 0, st>>>(w);
 }
 void launch_tonemap(const Accumulators& acc, int mode, int npix, float samples, int op, uint8_t* rgb8, float* mean,
                     cudaStream_t st) {

@@ -114,6 +114,9 @@ static constexpr int kCounterLoopLimit = 57;
 static constexpr int kCounterIterTotal = 58;
 static constexpr int kCounterPixels = 41;
 static constexpr int kCounterPathTicket = 59;   // blocks of the path kernel that are done (0 between launches)
+// Ray total of the table's first row after the last pass (two words, written by
+// k_advance): the words from kCounterStackDrops to here are what a renderer reads back.
+static constexpr int kCounterRowRays = 60;
 static constexpr int kCounterWords = 64;
 
 // Iteration of a stage launched with `bounce` (-1 under path regeneration: read from the
