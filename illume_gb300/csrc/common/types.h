@@ -96,7 +96,7 @@ struct alignas(16) DevInstance {
 };
 static_assert(sizeof(DevInstance) == 128, "instance record must be 128 bytes");
 
-struct DevSphere { float cx, cy, cz, r; int material; int pad[3]; };
+struct alignas(16) DevSphere { float cx, cy, cz, r; int material; int pad[3]; };
 
 struct DevMaterial {
   int type, albedo_tex, roughness_tex, medium;
