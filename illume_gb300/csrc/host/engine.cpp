@@ -291,7 +291,9 @@ int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
   }
   launch_raygen(w, grid_raygen, st);
   for (int b = 0; b < depth; ++b) {
-    if (hand_over(b)) launch_paths(w, knobs, b, depth, kPathTail, nee ? grid_paths_nee : grid_paths, st, nee);
+    if (hand_over(b))
+      launch_paths(w, knobs, b, depth, knobs.overlap ? kPathTailOverlap : kPathTail,
+                   nee ? grid_paths_nee : grid_paths, st, nee);
     launch_trace(w, knobs, b, grid_trace, st);
     launch_shade(w, knobs, b, nee ? grid_shade_nee : grid_shade, st, nee);
     if (nee) launch_shadow(w, knobs, b, grid_shadow, st);

@@ -145,9 +145,14 @@ static constexpr int kDefaultRayGroup = 16;
 // device several times over (311,296 lanes at 64 registers). Hand-over at 2^16 / 2^17 /
 // 2^18 / 2^19 rays: textured scene 2.54 / 2.19 / 2.21 / 2.37 ms, light sampling 7.02 /
 // 7.17 / 7.18 / 7.59, 16 large meshes 5.65 / 5.63 / 5.62 / 5.89.
+// Where passes of other tables run beside it the path kernel holds registers they could
+// use: there a larger pass hands over at 3 * 2^15 rays, 32 to a warp (light sampling 6.90
+// -> 6.68 ms, a textured render of 6M paths 5.00 -> 4.83, instances 3.36 -> 3.23, served
+// mixes 0.66 -> 0.61 and 1.50 -> 1.42; at 2^16 16 large meshes lose 5%).
 static constexpr int kPathBlocks = 4;
 static constexpr int kPathPass = 1 << 18;
 static constexpr int kPathTail = 1 << 17;
+static constexpr int kPathTailOverlap = 3 << 15;
 
 // Settings shared by every job of a table (they select kernel instances).
 struct RenderKnobs {

@@ -14,7 +14,8 @@
 // contributions are added in bounce order, so the image does not depend on the choice.
 //
 // Bound: latency. A warp's step costs the longest search of its lanes, so when there are
-// fewer paths than lanes they are spread over the warps (`width` lanes of each).
+// fewer paths than lanes they are spread over the warps (`width` lanes of each; `spread`),
+// unless other tables' passes want the registers of the warps that this saves.
 #include <algorithm>
 
 #include "launch.h"
@@ -24,7 +25,7 @@
 namespace illume {
 
 template <bool NEE, int ISECT>
-__global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int bounce, int depth, int limit) {
+__global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int bounce, int depth, int limit, int spread) {
   const unsigned FULL = 0xffffffffu;
   const bool start = bounce < 0;
   const int parity = start ? 0 : bounce & 1;
@@ -33,7 +34,7 @@ __global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int b
   int* fetch = w.counters + 44 + parity;   // zero here: set by the pass plan or the last trace stage
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
-  const int width = min(32, (n + warps - 1) / warps);
+  const int width = spread ? min(32, (n + warps - 1) / warps) : 32;
   int stack[kStack];
   float4 qo = make_float4(0, 0, 0, 0), qd = qo, qt = qo;
   int b = 0, job = -1;
@@ -140,7 +141,8 @@ const void* paths_kernel_ptr(int isect, bool nee) {
 
 void launch_paths(const WaveBuffers& w, const RenderKnobs& k, int bounce, int depth, int limit, int grid,
                   cudaStream_t st, bool nee) {
-  void* args[] = {const_cast<WaveBuffers*>(&w), &bounce, &depth, &limit};
+  int spread = k.overlap ? 0 : 1;
+  void* args[] = {const_cast<WaveBuffers*>(&w), &bounce, &depth, &limit, &spread};
   cudaLaunchKernel(paths_kernel_ptr(k.isect, nee), dim3(grid), dim3(128), args, 0, st);
 }
 

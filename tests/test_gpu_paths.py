@@ -72,3 +72,19 @@ def test_jobs_of_different_depths_share_a_table():
         assert np.array_equal(got["mean"], ref["mean"], equal_nan=True) and got["stats"].rays == ref["stats"].rays
         r.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("kind", ["ground", "medium"])
+def test_overlapping_engines_hand_over_too(kind):
+    ctx = Context(0)
+    sc = HostScene.from_data(ctx, scene(kind))
+    out = []
+    for bvh, engines in ((C.BVH_BINARY, 1), (C.BVH_WIDE4, 2), (C.BVH_WIDE4, 4)):
+        r = Renderer(ctx, sc, spp=8, max_depth=11, width=512, height=300, accum_mode=C.ACCUM_FP64, bvh_kind=bvh,
+                     engines=engines)
+        o = r.render(sums=True)
+        out.append((o["sum"], o["stats"].rays))
+        r.close()
+    for s, n in out[1:]:
+        assert n == out[0][1] and np.array_equal(s, out[0][0], equal_nan=True)
+    ctx.close()
