@@ -81,9 +81,9 @@ struct DevMesh {
   const float* positions;       // 3 floats per vertex
   const float* normals;         // 3 floats per vertex or null (face normals)
   const float* texcoords;       // 2 floats per vertex or null
+  const float4* face_normals;   // one per triangle, for meshes without normals (null: computed where needed)
   int num_tris;
   int bvh2_root_leaf;           // 1 if the whole mesh is one leaf (no inner node)
-  int pad[2];
 };
 
 // 128 bytes on a 16-byte boundary, read as 16-byte words: the box, mesh and material in two

@@ -1,5 +1,7 @@
 #include "runtime.h"
 
+#include "../kernels/launch.h"
+
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -470,6 +472,28 @@ int Scene::build_and_upload(std::string* err) {
     if (h.mesh_has_texcoords[i]) UP(h.texcoords.data() + 2 * vo, 2 * sizeof(float) * V, m.texcoords);
     m.num_tris = h.mesh_num_tris[i];
     m.bvh2_root_leaf = b.root_leaf ? 1 : 0;
+  }
+  // face normals of the meshes without normals (16 bytes per triangle, made on the device
+  // by the arithmetic of shading), where there is memory to spare: a context with a budget
+  // leaves it to its owner, and shading computes a normal whose mesh has none
+  size_t flat = 0;
+  for (int i = 0; i < nm; ++i)
+    if (!h.mesh_has_normals[i]) flat += (size_t)h.mesh_num_tris[i];
+  if (flat && !ctx->budget) {
+    std::unique_ptr<DevBuffer> fn(new DevBuffer);
+    if (fn->alloc(ctx, sizeof(float4) * flat) == ILLUME_OK) {
+      float4* at = fn->as<float4>();
+      for (int i = 0; i < nm; ++i) {
+        if (h.mesh_has_normals[i]) continue;
+        launch_face_normals(meshes[i].tris, meshes[i].positions, h.mesh_num_tris[i], at, ctx->stream);
+        meshes[i].face_normals = at;
+        at += h.mesh_num_tris[i];
+      }
+      device_bytes += fn->size();
+      buffers.push_back(std::move(fn));
+    } else {
+      cudaGetLastError();
+    }
   }
   const int ni = (int)h.inst_mesh.size();
   std::vector<DevInstance>& inst = t_instances;

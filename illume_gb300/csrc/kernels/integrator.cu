@@ -403,6 +403,14 @@ __global__ void k_clear(Accumulators acc, int npix) {
   }
 }
 
+// Face normals of a mesh without normals, made once when it is uploaded.
+__global__ void __launch_bounds__(256) k_face_normals(const int* tris, const float* positions, int n, float4* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const V3 f = face_normal(positions, tris[3 * i], tris[3 * i + 1], tris[3 * i + 2]);
+  out[i] = make_float4(f.x, f.y, f.z, 0.0f);
+}
+
 // BSDF test hook: layout of illume_bsdf_batch (include/illume.h).
 struct FixedRng {
   float u[3];
@@ -486,6 +494,9 @@ void launch_tonemap(const Accumulators& acc, int mode, int npix, float samples, 
 void launch_clear_accumulators(const Accumulators& acc, int npix, cudaStream_t st) {
   const int grid = (3 * npix + 255) / 256;
   if (grid > 0) k_clear<<<grid < 4096 ? grid : 4096, 256, 0, st>>>(acc, npix);
+}
+void launch_face_normals(const int* tris, const float* positions, int n, float4* out, cudaStream_t st) {
+  if (n > 0) k_face_normals<<<(n + 255) / 256, 256, 0, st>>>(tris, positions, n, out);
 }
 void launch_bsdf_batch(int type, int dist, const float* in, int n, float* out, cudaStream_t st) {
   if (n > 0) k_bsdf_batch<<<(n + 127) / 128, 128, 0, st>>>(type, dist, in, n, out);

@@ -196,6 +196,8 @@ void launch_tonemap(const Accumulators& acc, int accum_mode, int npix, float sam
                     float* mean, cudaStream_t st);
 void launch_clear_accumulators(const Accumulators& acc, int npix, cudaStream_t st);
 
+void launch_face_normals(const int* tris, const float* positions, int n, float4* out, cudaStream_t st);
+
 // test hooks
 // d_view: a device copy of sc (read by the persistent 8-wide kernel, bvh_kind 2)
 void launch_trace_hook(const SceneView& sc, const SceneView* d_view, const float* rays8, int n, int isect,
