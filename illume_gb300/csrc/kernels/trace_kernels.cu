@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(128) k_trace_sm(WaveBuffers w, const SceneView
 // longest search, so rays that do not fill the device are spread over more warps. Blocks
 // of 64 give a finished block's place to the next one sooner than blocks of 128.
 // 3M unordered rays on 16 meshes (500k triangles): 5.19 ms with the compiler's registers,
-// exact reciprocals and instances in index order, 2.44 ms with the default trace kernel's
+// exact reciprocals and instances in index order, 2.32 ms with the default trace kernel's
 // settings. FEW: at most 102 registers for batches that do not fill the device at 64, where
 // latency counts (1,000 rays 192 -> 41 us, 20,000 on one mesh 74 -> 66, 100,000 97 -> 90;
 // at 64 registers 45, 82 and 109).
