@@ -10,6 +10,8 @@ namespace illume {
 Engine::~Engine() {
   drop_graphs();
   if (side) cudaStreamDestroy(side);
+  if (side_start) cudaEventDestroy(side_start);
+  if (side_done) cudaEventDestroy(side_done);
 }
 
 void Engine::drop_graphs() {
@@ -80,6 +82,13 @@ int Engine::ensure_shadow(std::string* err) {
     grid_shade_nee = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant, true), 128, ctx->device);
     grid_paths_nee = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, true), 128, ctx->device);
   }
+  auto fork_join = [&]() -> int {   // what the occlusion launches beside the next bounce need
+    if (!side) ILLUME_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    if (!side_start) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_start, cudaEventDisableTiming));
+    if (!side_done) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_done, cudaEventDisableTiming));
+    return ILLUME_OK;
+  };
+  if (const int fj = fork_join(); fj != ILLUME_OK) { *err = last_error(); return fj; }
   if (s_orig.get() && s_orig.size() >= sizeof(float4) * (size_t)qcap) return ILLUME_OK;
   int st;
   if ((st = s_orig.alloc(ctx, sizeof(float4) * (size_t)qcap)) != ILLUME_OK) { *err = last_error(); return st; }
@@ -290,14 +299,36 @@ int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
     return ILLUME_OK;
   }
   launch_raygen(w, grid_raygen, st);
+  // A bounce's occlusion rays run beside the next bounce's closest-hit rays: the two read
+  // different queues and counters, and only shading (and the path kernel) needs both done,
+  // since a path's contributions are added in bounce order. Each launch's last rays leave
+  // most of the device to the other. Next-event renders, ms on the device: ground 512x512 x
+  // 32 samples 6.64 -> 6.42, Cornell box 256x256 x 32 2.72 -> 2.57, 16 meshes 6.97 -> 6.75,
+  // textured 10.48 -> 10.05 (the closest-hit launch captured first: Cornell box 2.67).
+  bool beside = false;
+  auto join = [&]() -> cudaError_t {
+    if (!beside) return cudaSuccess;
+    beside = false;
+    const cudaError_t e = cudaEventRecord(side_done, side);
+    return e == cudaSuccess ? cudaStreamWaitEvent(st, side_done, 0) : e;
+  };
   for (int b = 0; b < depth; ++b) {
-    if (hand_over(b))
+    if (hand_over(b)) {
+      ILLUME_CUDA_TRY(join());
       launch_paths(w, knobs, b, depth, knobs.overlap ? kPathTailOverlap : kPathTail,
                    nee ? grid_paths_nee : grid_paths, st, nee);
+    }
     launch_trace(w, knobs, b, grid_trace, st);
+    ILLUME_CUDA_TRY(join());
     launch_shade(w, knobs, b, nee ? grid_shade_nee : grid_shade, st, nee);
-    if (nee) launch_shadow(w, knobs, b, grid_shadow, st);
+    if (nee) {
+      ILLUME_CUDA_TRY(cudaEventRecord(side_start, st));
+      ILLUME_CUDA_TRY(cudaStreamWaitEvent(side, side_start, 0));
+      launch_shadow(w, knobs, b, grid_shadow, side);
+      beside = true;
+    }
   }
+  ILLUME_CUDA_TRY(join());
   return ILLUME_OK;
 }
 

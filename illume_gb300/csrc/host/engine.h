@@ -37,7 +37,8 @@ struct Engine {
   int grid_trace = 0, grid_shade = 0, grid_raygen = 0, grid_acc = 0, grid_shadow = 0, grid_shade_nee = 0;
   int grid_paths = 0, grid_paths_nee = 0;
   cudaStream_t stream = nullptr;            // the engine's stream (the context's unless set before init)
-  cudaStream_t side = nullptr;              // captures the regeneration loop's body
+  cudaStream_t side = nullptr;              // captures the regeneration loop's body and the occlusion launches
+  cudaEvent_t side_start = nullptr, side_done = nullptr;   // fork and join of the occlusion rays
   std::map<int, cudaGraphExec_t> graphs;   // captured pass by (depth, path kernel alone, shadow stage)
   std::map<int, cudaGraphExec_t> head_graphs;   // the same without accumulate and advance
   cudaGraphExec_t acc_graph = nullptr;          // accumulate + advance
