@@ -76,19 +76,21 @@ static int capture_while(cudaStream_t st, cudaStream_t side, const std::function
   return ILLUME_OK;
 }
 
+// What a pass forks with: its second half, or occlusion launches beside the next bounce.
+int Engine::ensure_side() {
+  if (!side) ILLUME_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  if (!side_start) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_start, cudaEventDisableTiming));
+  if (!side_done) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_done, cudaEventDisableTiming));
+  return ILLUME_OK;
+}
+
 int Engine::ensure_shadow(std::string* err) {
   if (!grid_shadow) {   // the next-event kernels' grids, looked up by the tables that use them
     grid_shadow = kernel_grid_blocks(shadow_kernel_ptr(knobs.bvh_kind), 128, ctx->device);
     grid_shade_nee = kernel_grid_blocks(shade_kernel_ptr(knobs.shade_variant, true), 128, ctx->device);
     grid_paths_nee = kernel_grid_blocks(paths_kernel_ptr(knobs.isect, true), 128, ctx->device);
   }
-  auto fork_join = [&]() -> int {   // what the occlusion launches beside the next bounce need
-    if (!side) ILLUME_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-    if (!side_start) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_start, cudaEventDisableTiming));
-    if (!side_done) ILLUME_CUDA_TRY(cudaEventCreateWithFlags(&side_done, cudaEventDisableTiming));
-    return ILLUME_OK;
-  };
-  if (const int fj = fork_join(); fj != ILLUME_OK) { *err = last_error(); return fj; }
+  if (const int fj = ensure_side(); fj != ILLUME_OK) { *err = last_error(); return fj; }
   if (s_orig.get() && s_orig.size() >= sizeof(float4) * (size_t)qcap) return ILLUME_OK;
   int st;
   if ((st = s_orig.alloc(ctx, sizeof(float4) * (size_t)qcap)) != ILLUME_OK) { *err = last_error(); return st; }
@@ -170,13 +172,14 @@ int Engine::init(Context* c, int nrows, int ncap, const RenderKnobs& k, std::str
   int st;
   if ((st = alloc_paths(err)) != ILLUME_OK) return st;
 #define ALLOC(buf, bytes) if ((st = (buf).alloc(ctx, (bytes))) != ILLUME_OK) { *err = last_error(); return st; }
-  ALLOC(counters, sizeof(int) * kCounterWords);
+  ALLOC(counters, sizeof(int) * kCounterWords * (halves ? 2 : 1));
   ALLOC(rays, sizeof(unsigned long long));
   ALLOC(visits, 3 * sizeof(unsigned long long));
   ALLOC(jobs, sizeof(JobDesc) * (size_t)rows);
   ALLOC(path_base, sizeof(int) * (size_t)(rows + 1));
   ALLOC(pixel_base, sizeof(int) * (size_t)(rows + 1));
 #undef ALLOC
+  if (halves && (st = ensure_side()) != ILLUME_OK) { *err = last_error(); return st; }
   mirror.assign(rows, JobDesc{});
   ILLUME_CUDA_TRY(cudaMemsetAsync(counters.get(), 0, counters.size(), stream));
   ILLUME_CUDA_TRY(cudaMemsetAsync(rays.get(), 0, rays.size(), stream));
@@ -286,7 +289,7 @@ void Engine::launch_iteration(cudaStream_t st, cudaGraphConditionalHandle cond, 
 // every path, then depth x (trace, shade); with it: the first batch of paths, then a
 // while node that iterates until every path has ended (called inside a capture).
 int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
-  launch_plan(w, st);
+  launch_plan(split_pass() ? half(0) : w, st);
   if (regen) {
     launch_regen_start(w, st);
     launch_regen(w, grid_raygen, st);
@@ -298,7 +301,56 @@ int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
     launch_paths(w, knobs, -1, depth, 0, nee ? grid_paths_nee : grid_paths, st, nee);
     return ILLUME_OK;
   }
+  if (split_pass()) {   // never a path pass: kSplitPass > kPathPass
+    // The halves share nothing but the radiance slots, of which each path has its own, so
+    // the image does not depend on the split; the accumulation takes the whole pass.
+    const int grid = std::max(1, grid_raygen / 2);
+    ILLUME_CUDA_TRY(cudaEventRecord(side_start, st));
+    ILLUME_CUDA_TRY(cudaStreamWaitEvent(side, side_start, 0));
+    for (int h = 0; h < 2; ++h) {
+      const WaveBuffers x = half(h);
+      launch_raygen(x, grid, h ? side : st);
+      const int s = launch_bounces(x, h ? side : st, depth, nee, false);
+      if (s != ILLUME_OK) return s;
+    }
+    ILLUME_CUDA_TRY(cudaEventRecord(side_done, side));
+    ILLUME_CUDA_TRY(cudaStreamWaitEvent(st, side_done, 0));
+    return ILLUME_OK;
+  }
   launch_raygen(w, grid_raygen, st);
+  return launch_bounces(w, st, depth, nee, nee);
+}
+
+// Half h of the pass: its paths, in the queues' lower or upper part, with its own counters.
+WaveBuffers Engine::half(int h) const {
+  WaveBuffers x = w;
+  const int low = qcap / 2;
+  x.part = 1 + h;
+  x.qcap = h ? qcap - low : low;
+  if (h) {
+    for (int k = 0; k < 2; ++k) {
+      x.q_orig[k] += low;
+      x.q_dir[k] += low;
+      x.q_thr[k] += low;
+    }
+    x.hit += low;
+    x.hit_geom += low;
+    x.evq += (size_t)low * EV_COUNT;
+    x.counters += kCounterWords;
+    if (x.s_orig) {
+      x.s_orig += low;
+      x.s_dir += low;
+      x.s_val += low;
+    }
+  }
+  return x;
+}
+
+// depth x (trace, shade) of the rays queued in x. With `beside_next` the occlusion launches go to
+// the side stream.
+int Engine::launch_bounces(const WaveBuffers& x, cudaStream_t st, int depth, bool nee, bool beside_next) {
+  RenderKnobs k = knobs;
+  if (x.part) k.overlap = 1;
   // A bounce's occlusion rays run beside the next bounce's closest-hit rays: the two read
   // different queues and counters, and only shading (and the path kernel) needs both done,
   // since a path's contributions are added in bounce order. Each launch's last rays leave
@@ -315,16 +367,17 @@ int Engine::launch_head(cudaStream_t st, int depth, bool nee) {
   for (int b = 0; b < depth; ++b) {
     if (hand_over(b)) {
       ILLUME_CUDA_TRY(join());
-      launch_paths(w, knobs, b, depth, knobs.overlap ? kPathTailOverlap : kPathTail,
+      launch_paths(x, k, b, depth, k.overlap ? kPathTailOverlap : kPathTail,
                    nee ? grid_paths_nee : grid_paths, st, nee);
     }
-    launch_trace(w, knobs, b, grid_trace, st);
+    launch_trace(x, k, b, grid_trace, st);
     ILLUME_CUDA_TRY(join());
-    launch_shade(w, knobs, b, nee ? grid_shade_nee : grid_shade, st, nee);
-    if (nee) {
+    launch_shade(x, k, b, nee ? grid_shade_nee : grid_shade, st, nee);
+    if (nee && !beside_next) launch_shadow(x, k, b, grid_shadow, st);
+    if (beside_next) {
       ILLUME_CUDA_TRY(cudaEventRecord(side_start, st));
       ILLUME_CUDA_TRY(cudaStreamWaitEvent(side, side_start, 0));
-      launch_shadow(w, knobs, b, grid_shadow, side);
+      launch_shadow(x, k, b, grid_shadow, side);
       beside = true;
     }
   }
@@ -336,7 +389,7 @@ int Engine::launch_pass(cudaStream_t st, int depth, bool nee) {
   const int s = launch_head(st, depth, nee);
   if (s != ILLUME_OK) return s;
   launch_accumulate(w, grid_acc, st);
-  launch_advance(w, st);
+  launch_advance(split_pass() ? half(0) : w, st);
   return ILLUME_OK;
 }
 

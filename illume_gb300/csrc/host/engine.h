@@ -28,6 +28,7 @@ struct Engine {
   int ray_group = kDefaultRayGroup;   // samples of a pixel together in the camera-ray queue
   float regen_threshold = 1.0f;
   bool regen = false;
+  bool halves = false;     // large passes run as two halves side by side (set before init; one row, no regeneration)
   RenderKnobs knobs{};
   DevBuffer q_orig[2], q_dir[2], q_thr[2], q_bounce[2], hit, hit_geom, evq, counters, contrib, rays, visits;
   DevBuffer jobs, path_base, pixel_base;
@@ -37,8 +38,8 @@ struct Engine {
   int grid_trace = 0, grid_shade = 0, grid_raygen = 0, grid_acc = 0, grid_shadow = 0, grid_shade_nee = 0;
   int grid_paths = 0, grid_paths_nee = 0;
   cudaStream_t stream = nullptr;            // the engine's stream (the context's unless set before init)
-  cudaStream_t side = nullptr;              // captures the regeneration loop's body and the occlusion launches
-  cudaEvent_t side_start = nullptr, side_done = nullptr;   // fork and join of the occlusion rays
+  cudaStream_t side = nullptr;              // captures the regeneration loop's body, the occlusion launches, a pass's second half
+  cudaEvent_t side_start = nullptr, side_done = nullptr;   // fork and join of the side stream
   std::map<int, cudaGraphExec_t> graphs;   // captured pass by (depth, path kernel alone, shadow stage)
   std::map<int, cudaGraphExec_t> head_graphs;   // the same without accumulate and advance
   cudaGraphExec_t acc_graph = nullptr;          // accumulate + advance
@@ -79,9 +80,9 @@ struct Engine {
   // Launches of the next pass with `depth` bounces.
   int launches_per_pass(int depth, bool nee = false) const {
     if (path_pass(depth)) return 5;
-    int n = 5 + (nee ? 3 : 2) * depth;
+    int n = 1 + (nee ? 3 : 2) * depth;
     for (int b = 2; b < depth; ++b) n += hand_over(b);
-    return n;
+    return 4 + (split_pass() ? 2 : 1) * n;
   }
   // Launches of regenerating passes with `iterations` loop iterations in all.
   static long long launches_regen(long long passes, long long iterations, bool nee = false) {
@@ -92,6 +93,7 @@ struct Engine {
 
  private:
   int alloc_paths(std::string* err);
+  int ensure_side();
   void point();
   void advance_mirror();
   // Whether the next pass is small enough to run as one path-kernel launch. (With depth 0
@@ -104,7 +106,14 @@ struct Engine {
   // the Cornell box (256x256, 64 samples) lost 1.5%, at the powers of two from 2 nothing,
   // and the other scenes were within 2% of either.
   bool hand_over(int b) const { return paths_kernel_for(knobs) && !regen && b >= 2 && (b & (b - 1)) == 0; }
-  int graph_key(int depth, bool nee) const { return 4 * depth + (path_pass(depth) ? 2 : 0) + (nee ? 1 : 0); }
+  // Whether the next pass runs as two halves of its paths, each through its own queues and
+  // counters on its own stream (launch_head).
+  bool split_pass() const { return halves && !regen && paths_in_pass() >= kSplitPass; }
+  int graph_key(int depth, bool nee) const {
+    return 8 * depth + (split_pass() ? 4 : 0) + (path_pass(depth) ? 2 : 0) + (nee ? 1 : 0);
+  }
+  WaveBuffers half(int h) const;
+  int launch_bounces(const WaveBuffers& x, cudaStream_t st, int depth, bool nee, bool beside);
   int launch_head(cudaStream_t st, int depth, bool nee);
   int launch_pass(cudaStream_t st, int depth, bool nee);
   void launch_iteration(cudaStream_t st, cudaGraphConditionalHandle cond, bool use_cond, int depth, bool nee);

@@ -71,18 +71,22 @@ __global__ void __launch_bounds__(1024) k_plan(WaveBuffers w) {
     const int paths = over ? 0 : (int)carry[0], pixels = over ? 0 : (int)carry[1];
     w.job_path_base[w.njobs] = paths;
     w.job_pixel_base[w.njobs] = pixels;
-    w.counters[kCounterPaths] = paths;
     w.counters[kCounterPixels] = pixels;
-    w.counters[0] = paths;
-    w.counters[1] = 0;
-    w.counters[44] = 0;   // trace ray-fetch counters by bounce parity
-    w.counters[45] = 0;
-    w.counters[46] = 0;   // shadow-ray counts by bounce parity
-    w.counters[47] = 0;
-    w.counters[48] = 0;   // shadow-ray fetch counters by bounce parity
-    w.counters[49] = 0;
     if (over) w.counters[42] = 1;
-    for (int c = 0; c < EV_COUNT; ++c) ev_counts(w, 0)[c] = 0;
+    const int first = w.part ? paths / 2 : paths;
+    for (int h = 0; h < (w.part ? 2 : 1); ++h) {
+      int* n = w.counters + h * kCounterWords;
+      n[kCounterPaths] = paths;
+      n[0] = h ? paths - first : first;
+      n[1] = 0;
+      n[44] = 0;   // trace ray-fetch counters by bounce parity
+      n[45] = 0;
+      n[46] = 0;   // shadow-ray counts by bounce parity
+      n[47] = 0;
+      n[48] = 0;   // shadow-ray fetch counters by bounce parity
+      n[49] = 0;
+      for (int c = 0; c < EV_COUNT; ++c) n[2 + c] = 0;
+    }
   }
 }
 
@@ -98,8 +102,10 @@ __device__ __forceinline__ void start_path(const WaveBuffers& w, int i, int q, i
 }
 
 __global__ void __launch_bounds__(256) k_raygen(WaveBuffers w) {
-  const int total = w.counters[kCounterPaths];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) start_path(w, i, i, 0);
+  const int total = w.counters[0];   // the whole pass's paths, or one half's
+  const int first = w.part == 2 ? w.counters[kCounterPaths] - total : 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    start_path(w, first + i, i, 0);
 }
 
 // ---- path regeneration (see launch.h) ----
@@ -335,7 +341,11 @@ __global__ void k_advance(WaveBuffers w) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= w.njobs) return;
   JobDesc& J = w.jobs[j];
-  if (j == 0) *reinterpret_cast<unsigned long long*>(w.counters + kCounterRowRays) = J.rays;
+  if (j == 0) {
+    *reinterpret_cast<unsigned long long*>(w.counters + kCounterRowRays) = J.rays;
+    // a second half's overflow flag, where a renderer looks for the pass's
+    if (w.part && w.counters[kCounterWords + kCounterStackDrops]) w.counters[kCounterStackDrops] = 1;
+  }
   if (J.nsamples <= 0) return;
   advance_pass_state(J.sample_base, J.nsamples, J.sample_end, J.per_pass, J.flags);
 }

@@ -89,6 +89,7 @@ struct WaveBuffers {
 
   int cap;               // path slots of one pass (per-path radiance)
   int qcap;              // queue slots (rays in flight); equal to cap without regeneration
+  int part;              // 0: the whole pass; 1, 2: its first and second half of paths (Engine::halves)
 };
 
 // counters[]: [0..1] queue sizes by parity, [2 + 16 * parity + class] event counts,
@@ -117,7 +118,7 @@ static constexpr int kCounterPathTicket = 59;   // blocks of the path kernel tha
 // Ray total of the table's first row after the last pass (two words, written by
 // k_advance): the words from kCounterStackDrops to here are what a renderer reads back.
 static constexpr int kCounterRowRays = 60;
-static constexpr int kCounterWords = 64;
+static constexpr int kCounterWords = 64;        // a second half's counters follow the first's
 
 // Iteration of a stage launched with `bounce` (-1 under path regeneration: read from the
 // counters), and the bounce of queued ray i.
@@ -150,6 +151,7 @@ static constexpr int kDefaultRayGroup = 16;
 // -> 6.68 ms, a textured render of 6M paths 5.00 -> 4.83, instances 3.36 -> 3.23, served
 // mixes 0.66 -> 0.61 and 1.50 -> 1.42; at 2^16 16 large meshes lose 5%).
 static constexpr int kPathBlocks = 4;
+static constexpr int kSplitPass = 1 << 20;   // paths from which a pass may run as two halves (Renderer::init)
 static constexpr int kPathPass = 1 << 18;
 static constexpr int kPathTail = 1 << 17;
 static constexpr int kPathTailOverlap = 3 << 15;

@@ -187,7 +187,9 @@ typedef struct {
   int32_t engines;            /* renderer: engines (path tables on their own streams) taking
                                * turns on the passes of a call, so that one pass's last bounces
                                * overlap the next passes; 0 = for a pass of 4M paths or more one
-                               * per 16M paths, 2 to 4, else 1; at most 16 and at most the
+                               * per 16M paths, 2 to 4, else 1 (a pass of 1M paths or more in a
+                               * scene without an environment then runs as two halves side by
+                               * side on that engine; not with 1); at most 16 and at most the
                                * samples per pass.
                                * The image does not depend on it. The server ignores it
                                * (ILLUME_SERVER_LANES). */
