@@ -240,18 +240,18 @@ int Engine::set_trace_variant(int variant) {
   return ILLUME_OK;
 }
 
+// Both take the mirror's values now, as launch arguments: advance_mirror changes the mirror
+// while the work queued before may still run, and a copy from ordinary host memory may read
+// its source as late as that (integrated CPU memory is read in place).
 int Engine::write_row(int r) {
-  ILLUME_CUDA_TRY(cudaMemcpyAsync(jobs.as<JobDesc>() + r, &mirror[r], sizeof(JobDesc), cudaMemcpyHostToDevice,
-                                  stream));
+  ILLUME_CUDA_TRY(launch_write_row(jobs.as<JobDesc>() + r, mirror[r], stream));
   return ILLUME_OK;
 }
 
 int Engine::write_pass_state(int r) {
-  const size_t off = offsetof(JobDesc, sample_base);
-  static_assert(offsetof(JobDesc, per_pass) == offsetof(JobDesc, sample_base) + 3 * sizeof(int), "pass state words");
-  ILLUME_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char*>(jobs.as<JobDesc>() + r) + off,
-                                  reinterpret_cast<const char*>(&mirror[r]) + off, 4 * sizeof(int),
-                                  cudaMemcpyHostToDevice, stream));
+  const JobDesc& J = mirror[r];
+  ILLUME_CUDA_TRY(launch_write_pass_state(jobs.as<JobDesc>() + r,
+                                          make_int4(J.sample_base, J.nsamples, J.sample_end, J.per_pass), stream));
   return ILLUME_OK;
 }
 

@@ -413,6 +413,14 @@ __global__ void k_clear(Accumulators acc, int npix) {
   }
 }
 
+__global__ void k_write_row(JobDesc* dst, JobDesc row) { *dst = row; }
+__global__ void k_write_pass_state(JobDesc* dst, int4 s) {
+  dst->sample_base = s.x;
+  dst->nsamples = s.y;
+  dst->sample_end = s.z;
+  dst->per_pass = s.w;
+}
+
 // Face normals of a mesh without normals, made once when it is uploaded.
 __global__ void __launch_bounds__(256) k_face_normals(const int* tris, const float* positions, int n, float4* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -504,6 +512,15 @@ void launch_tonemap(const Accumulators& acc, int mode, int npix, float samples, 
 void launch_clear_accumulators(const Accumulators& acc, int npix, cudaStream_t st) {
   const int grid = (3 * npix + 255) / 256;
   if (grid > 0) k_clear<<<grid < 4096 ? grid : 4096, 256, 0, st>>>(acc, npix);
+}
+cudaError_t launch_write_row(JobDesc* dst, const JobDesc& row, cudaStream_t st) {
+  JobDesc r = row;
+  void* args[] = {&dst, &r};
+  return cudaLaunchKernel((const void*)k_write_row, dim3(1), dim3(1), args, 0, st);
+}
+cudaError_t launch_write_pass_state(JobDesc* dst, int4 state, cudaStream_t st) {
+  void* args[] = {&dst, &state};
+  return cudaLaunchKernel((const void*)k_write_pass_state, dim3(1), dim3(1), args, 0, st);
 }
 void launch_face_normals(const int* tris, const float* positions, int n, float4* out, cudaStream_t st) {
   if (n > 0) k_face_normals<<<(n + 255) / 256, 256, 0, st>>>(tris, positions, n, out);

@@ -167,6 +167,11 @@ struct RenderKnobs {
 
 int kernel_grid_blocks(const void* fn, int block, int device);
 
+// A job row, or its pass state (sample_base, nsamples, sample_end, per_pass), written from
+// the launch's arguments.
+cudaError_t launch_write_row(JobDesc* dst, const JobDesc& row, cudaStream_t st);
+cudaError_t launch_write_pass_state(JobDesc* dst, int4 state, cudaStream_t st);
+
 void launch_plan(const WaveBuffers& w, cudaStream_t st);
 void launch_raygen(const WaveBuffers& w, int grid, cudaStream_t st);
 // Path regeneration. A pass runs as a loop of iterations (trace, shade, [shadow], plan of
