@@ -438,14 +438,15 @@ int illume_trace_closest(illume_context* ctx, illume_scene* scene, const float* 
   const bool staged = ray_bytes + hit_bytes <= Context::kStagingBytes / 2;
   const void* from = rays;
   if (staged) from = memcpy(c.staging(), rays, ray_bytes);
-  ILLUME_CUDA_TRY(cudaMemcpyAsync(d_rays, from, ray_bytes, cudaMemcpyHostToDevice, c.stream));
-  if ((st = illume_trace_closest_device(ctx, scene, d_rays, n, intersector, bvh_kind, d_hits)) != ILLUME_OK) {
-    cudaStreamSynchronize(c.stream);   // the copy above is done with its source
-    return st;
-  }
   void* to = staged ? (void*)(c.staging() + ray_bytes) : (void*)hits;
-  ILLUME_CUDA_TRY(cudaMemcpyAsync(to, d_hits, hit_bytes, cudaMemcpyDeviceToHost, c.stream));
-  ILLUME_CUDA_TRY(cudaStreamSynchronize(c.stream));
+  ILLUME_CUDA_TRY(cudaMemcpyAsync(d_rays, from, ray_bytes, cudaMemcpyHostToDevice, c.stream));
+  st = illume_trace_closest_device(ctx, scene, d_rays, n, intersector, bvh_kind, d_hits);
+  cudaError_t e = cudaSuccess;
+  if (st == ILLUME_OK) e = cudaMemcpyAsync(to, d_hits, hit_bytes, cudaMemcpyDeviceToHost, c.stream);
+  const cudaError_t w = cudaStreamSynchronize(c.stream);   // after a failure too: the staging memory is free again
+  if (st != ILLUME_OK) return st;
+  ILLUME_CUDA_TRY(e);
+  ILLUME_CUDA_TRY(w);
   if (staged) memcpy(hits, to, hit_bytes);
   return ILLUME_OK;
 }

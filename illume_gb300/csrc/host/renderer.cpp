@@ -240,34 +240,57 @@ int Renderer::enqueue(bool accumulate, Call* call) {
   ILLUME_CUDA_TRY(cudaEventRecord(ev1, st));
   call->launched = -before;
   for (int e = 0; e < nengines; ++e) call->launched += engine(e).launches;
-  int* status = reinterpret_cast<int*>(ctx->staging());
-  for (int e = 0; e < nengines; ++e)
-    ILLUME_CUDA_TRY(cudaMemcpyAsync(status + e * kStatusWords, engine(e).w.counters + kStatusFirst,
-                                    sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, st));
+  if ((s = enqueue_status()) != ILLUME_OK) return s;
   samples_done += spp;
   next_sample += spp;
   return ILLUME_OK;
 }
 
-int Renderer::finish(const Call& call, illume_render_stats* stats) {
-  ILLUME_CUDA_TRY(cudaGetLastError());
+int Renderer::enqueue_status() {
+  int* status = reinterpret_cast<int*>(ctx->staging());
+  for (int e = 0; e < nengines; ++e)
+    ILLUME_CUDA_TRY(cudaMemcpyAsync(status + e * kStatusWords, engine(e).w.counters + kStatusFirst,
+                                    sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, ctx->stream));
+  return ILLUME_OK;
+}
+
+// Takes the status words that enqueue_status copied (after a wait): what the engines added
+// to their totals since the last time, and the flags.
+Renderer::Status Renderer::take_status() {
   const int* status = reinterpret_cast<const int*>(ctx->staging());
-  stack_overflow = false;
-  long long iters = 0;
-  int64_t rays = 0;
-  bool loop_limit = false;
+  Status t;
   for (int e = 0; e < nengines; ++e) {
     const int* c = status + e * kStatusWords - kStatusFirst;
     unsigned long long total;
     memcpy(&total, c + kCounterRowRays, sizeof(total));
-    stack_overflow = stack_overflow || c[kCounterStackDrops] != 0;
-    iters += (long long)c[kCounterIterTotal] - iter_total[e];
+    t.stack_drops = t.stack_drops || c[kCounterStackDrops] != 0;
+    t.loop_limit = t.loop_limit || c[kCounterLoopLimit] != 0;
+    t.iterations += (long long)c[kCounterIterTotal] - iter_total[e];
     iter_total[e] = c[kCounterIterTotal];
-    loop_limit = loop_limit || c[kCounterLoopLimit] != 0;
-    rays += (int64_t)(total - rays_total[e]);
+    t.rays += (int64_t)(total - rays_total[e]);
     rays_total[e] = total;
   }
-  if (loop_limit) {
+  return t;
+}
+
+// Ends a call that failed after it had queued work. The passes it launched still run, and
+// status words may be on their way into the staging memory, which the context's next call
+// uses: wait for all of it, and take the totals so that the next call's statistics leave
+// this one's rays out. The message of the failure stays.
+void Renderer::abandon() {
+  for (cudaStream_t x : more_streams) cudaStreamSynchronize(x);
+  cudaStreamSynchronize(ctx->stream);
+  cudaGetLastError();   // reported by the call that failed
+  const std::string message = last_error();
+  if (enqueue_status() == ILLUME_OK && cudaStreamSynchronize(ctx->stream) == cudaSuccess) take_status();
+  set_error(message);
+}
+
+int Renderer::finish(const Call& call, illume_render_stats* stats) {
+  ILLUME_CUDA_TRY(cudaGetLastError());
+  const Status t = take_status();
+  stack_overflow = t.stack_drops;
+  if (t.loop_limit) {
     samples_done -= p.spp;
     next_sample -= p.spp;
     set_error("a path-regeneration loop reached its iteration bound: the pass ended before all its paths");
@@ -276,11 +299,11 @@ int Renderer::finish(const Call& call, illume_render_stats* stats) {
   if (stats) {
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ev0, ev1);
-    stats->rays = rays;
+    stats->rays = t.rays;
     stats->paths = (int64_t)p.spp * npix;
     stats->render_ms = ms;
     const bool nee = p.estimator == ILLUME_ESTIMATOR_NEE;
-    stats->kernel_launches = eng.regen ? Engine::launches_regen(call.npasses, iters, nee) : call.launched;
+    stats->kernel_launches = eng.regen ? Engine::launches_regen(call.npasses, t.iterations, nee) : call.launched;
     stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - call.wall0).count();
     stats->h2d_bytes = 4 * sizeof(int);
     stats->d2h_bytes = kStatusWords * sizeof(int) * (size_t)nengines;
@@ -291,7 +314,7 @@ int Renderer::finish(const Call& call, illume_render_stats* stats) {
 int Renderer::render_device(bool accumulate, illume_render_stats* stats) {
   Call call;
   const int s = enqueue(accumulate, &call);
-  if (s != ILLUME_OK) return s;
+  if (s != ILLUME_OK) { abandon(); return s; }
   ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return finish(call, stats);
 }
@@ -304,10 +327,12 @@ int Renderer::render_and_read(float* mean, double* sum, double* sumsq_out, uint8
   }
   Call call;
   Outputs out;
-  if ((s = enqueue(false, &call)) != ILLUME_OK) return s;
-  if ((s = enqueue_read(mean, sum, sumsq_out, rgb8, &out)) != ILLUME_OK) return s;
+  if ((s = enqueue(false, &call)) != ILLUME_OK) { abandon(); return s; }
+  // (without memory for the outputs the render is done all the same, and is waited for)
+  const int read_status = enqueue_read(mean, sum, sumsq_out, rgb8, &out);
   ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if ((s = finish(call, stats)) != ILLUME_OK) return s;
+  if (read_status != ILLUME_OK) return read_status;
   finish_read(mean, sum, rgb8, out);
   return ILLUME_OK;
 }
@@ -416,8 +441,8 @@ void Renderer::finish_read(float* mean, double* sum, uint8_t* rgb8, const Output
 int Renderer::read(float* mean, double* sum, double* sumsq_out, uint8_t* rgb8) {
   Outputs o;
   const int s = enqueue_read(mean, sum, sumsq_out, rgb8, &o);
+  ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // after a failure too: a copy may be on its way
   if (s != ILLUME_OK) return s;
-  ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   finish_read(mean, sum, rgb8, o);
   return ILLUME_OK;
 }

@@ -58,7 +58,7 @@ struct Renderer {
 
  private:
   // A call in flight: launched by enqueue (its status copies go to the context's staging
-  // memory), ended by finish after a wait for the context's stream. enqueue_read /
+  // memory), ended by finish after a wait for the context's stream, or by abandon. enqueue_read /
   // finish_read do the same for the outputs; small mean / RGB8 images go through the
   // staging memory as well (one copy, none of them into pageable memory).
   struct Call {
@@ -70,7 +70,15 @@ struct Renderer {
     bool staged = false;
     std::vector<float> s32, c32;
   };
+  struct Status {
+    int64_t rays = 0;
+    long long iterations = 0;   // of the regeneration loop
+    bool stack_drops = false, loop_limit = false;
+  };
   int enqueue(bool accumulate, Call* call);
+  int enqueue_status();
+  Status take_status();
+  void abandon();
   int finish(const Call& call, illume_render_stats* stats);
   int enqueue_read(float* mean, double* sum, double* sumsq, uint8_t* rgb8, Outputs* out);
   void finish_read(float* mean, double* sum, uint8_t* rgb8, const Outputs& out);

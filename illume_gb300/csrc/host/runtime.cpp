@@ -48,6 +48,7 @@ int DevBuffer::alloc(Context* ctx, size_t bytes) {
   }
   cudaError_t e = cudaMalloc(&ptr_, bytes);
   if (e != cudaSuccess) {
+    cudaGetLastError();   // reported here, not by a later call's check
     ptr_ = nullptr;
     set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? ILLUME_ERR_OOM : ILLUME_ERR_CUDA;

@@ -295,9 +295,38 @@ static void pass_state() {
   illume_server_destroy(s);
 }
 
+// A render whose outputs cannot be allocated, or whose passes cannot all be launched, returns
+// with nothing of it left to run: the next call's staging memory and ray counts are its own.
+static void failed_render() {
+  World x;
+  for (int midway = 0; midway < 2; ++midway) {
+    illume_renderer* r = midway ? x.renderer(16, 16, 4, 1, 2) : x.renderer(16, 16, 4);
+    EXPECT(r);
+    if (!r) return;
+    std::vector<float> mean(3 * 256);
+    illume_render_stats st;
+    if (midway) g_fail_graph_launch = 2;              // the second pass's first graph
+    else x.ctx->c.budget = x.ctx->c.used.load() + 64; // no room for the output images
+    EXPECT(illume_render(r, mean.data(), nullptr, nullptr, nullptr, &st) == (midway ? ILLUME_ERR_CUDA : ILLUME_ERR_BUDGET));
+    x.ctx->c.budget = 0;
+    g_fail_graph_launch = -1;
+    EXPECT(g_queue.empty());
+    float rays[8] = {11, 0, 0, 0, 0, 0, 1, 0};
+    illume_hit hit;
+    memset(&hit, 0, sizeof(hit));
+    EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE4, &hit) == ILLUME_OK);
+    EXPECT(hit.t == 11.0f);
+    EXPECT(illume_render(r, mean.data(), nullptr, nullptr, nullptr, &st) == ILLUME_OK);
+    EXPECT(st.rays == 4 * kRaysPerSample);
+    EXPECT(mean[0] == 0.5f && mean[767] == 0.5f);
+    illume_renderer_destroy(r);
+  }
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
+  else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);
   return g_failed ? 1 : 0;
