@@ -76,6 +76,7 @@ static int finish_scene(illume_context* ctx, std::unique_ptr<illume_scene>& sc, 
   sc->s.ctx = &ctx->c;
   const int st = sc->s.build_and_upload(&err);
   if (st != ILLUME_OK) {
+    cudaStreamSynchronize(ctx->c.stream);   // copies from the scene's arrays, which go with it
     set_error(err.empty() ? std::string(last_error()) : err);
     return st;
   }

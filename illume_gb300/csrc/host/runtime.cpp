@@ -474,28 +474,6 @@ int Scene::build_and_upload(std::string* err) {
     m.num_tris = h.mesh_num_tris[i];
     m.bvh2_root_leaf = b.root_leaf ? 1 : 0;
   }
-  // face normals of the meshes without normals (16 bytes per triangle, made on the device
-  // by the arithmetic of shading), where there is memory to spare: a context with a budget
-  // leaves it to its owner, and shading computes a normal whose mesh has none
-  size_t flat = 0;
-  for (int i = 0; i < nm; ++i)
-    if (!h.mesh_has_normals[i]) flat += (size_t)h.mesh_num_tris[i];
-  if (flat && !ctx->budget) {
-    std::unique_ptr<DevBuffer> fn(new DevBuffer);
-    if (fn->alloc(ctx, sizeof(float4) * flat) == ILLUME_OK) {
-      float4* at = fn->as<float4>();
-      for (int i = 0; i < nm; ++i) {
-        if (h.mesh_has_normals[i]) continue;
-        launch_face_normals(meshes[i].tris, meshes[i].positions, h.mesh_num_tris[i], at, ctx->stream);
-        meshes[i].face_normals = at;
-        at += h.mesh_num_tris[i];
-      }
-      device_bytes += fn->size();
-      buffers.push_back(std::move(fn));
-    } else {
-      cudaGetLastError();
-    }
-  }
   const int ni = (int)h.inst_mesh.size();
   std::vector<DevInstance>& inst = t_instances;
   inst.assign(ni, DevInstance{});
@@ -625,6 +603,31 @@ int Scene::build_and_upload(std::string* err) {
     const int st_ = up(&view, sizeof(SceneView), &p_);
     if (st_ != ILLUME_OK) { *err = last_error(); return st_; }
     view_dev = reinterpret_cast<SceneView*>(p_);
+  }
+  // Face normals of the meshes without normals, made on the device by the arithmetic of
+  // shading, which computes a normal whose mesh has none. An extra: it comes after
+  // everything the scene cannot do without, takes at most a sixteenth of the memory that is
+  // left then, and leaves a context with a budget to its owner. (Positions and triangles
+  // never change after this, so illume_scene_upload, which copies them again, leaves the
+  // normals as they are.)
+  size_t flat = 0, left = 0, total = 0;
+  for (int i = 0; i < nm; ++i)
+    if (!h.mesh_has_normals[i]) flat += (size_t)h.mesh_num_tris[i];
+  if (flat && !ctx->budget && cudaMemGetInfo(&left, &total) == cudaSuccess && sizeof(float4) * flat <= left / 16) {
+    std::unique_ptr<DevBuffer> fn(new DevBuffer);
+    if (fn->alloc(ctx, sizeof(float4) * flat) == ILLUME_OK) {
+      float4* at = fn->as<float4>();
+      for (int i = 0; i < nm; ++i) {
+        if (h.mesh_has_normals[i]) continue;
+        launch_face_normals(meshes[i].tris, meshes[i].positions, h.mesh_num_tris[i], at, ctx->stream);
+        meshes[i].face_normals = at;
+        at += h.mesh_num_tris[i];
+      }
+      ILLUME_CUDA_TRY(cudaMemcpyAsync(const_cast<DevMesh*>(view.meshes), meshes.data(), sizeof(DevMesh) * (size_t)nm,
+                                      cudaMemcpyHostToDevice, ctx->stream));
+      device_bytes += fn->size();
+      buffers.push_back(std::move(fn));
+    }
   }
   ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   upload_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t1).count();

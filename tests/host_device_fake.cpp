@@ -193,12 +193,12 @@ struct World {
   illume_context* ctx = nullptr;
   illume_scene* scene = nullptr;
   int status;
-  World(int tris = 2) {
+  World(int tris = 2, int bitmap = 0) {
     illume_context_create(0, 0, &ctx);
-    status = load(tris);
+    status = load(tris, bitmap);
   }
-  // one instance of a strip of triangles without normals under a constant albedo
-  int load(int ntris) {
+  // one instance of a strip of triangles without normals; its albedo is constant, or a bitmap
+  int load(int ntris, int bitmap) {
     std::vector<float> P;
     std::vector<int32_t> T;
     for (int i = 0; i < ntris + 2; ++i) { P.push_back((float)(i / 2)); P.push_back((float)(i % 2)); P.push_back(0.0f); }
@@ -224,8 +224,13 @@ struct World {
     d.mat_medium = &air;
     d.mat_ior = d.mat_diffuse_fresnel = &one;
     d.mat_eta = d.mat_k = grey;
+    const int32_t type = bitmap ? ILLUME_TEX_BITMAP : ILLUME_TEX_CONSTANT, size = bitmap;
+    const std::vector<float> texels(4 * (size_t)bitmap * bitmap, 0.5f);
     d.num_textures = 1;
-    d.tex_type = d.tex_width = d.tex_height = d.tex_hdr = &zero;
+    d.tex_type = &type;
+    d.tex_width = d.tex_height = &size;
+    d.tex_hdr = &zero;
+    d.texels = texels.data();
     d.tex_color = d.tex_off = grey;
     d.tex_scale = scale;
     d.tex_texel_offset = &off;
@@ -295,6 +300,38 @@ static void pass_state() {
   illume_server_destroy(s);
 }
 
+// The table of face normals is an extra: a scene loads wherever there is memory for the
+// rest of it, and the table leaves most of what is left to the renders that follow.
+static void face_normal_memory() {
+  const int tris = 5000;
+  const size_t table = sizeof(float4) * tris;
+  size_t need;
+  {
+    World x(tris, 128);
+    EXPECT(x.status == ILLUME_OK && x.scene->s.t_meshes[0].face_normals);
+    need = g_used - table;
+  }
+  for (size_t spare : {(size_t)0, table, 15 * table, 16 * table}) {
+    g_limit = need + spare;
+    World x(tris, 128);
+    EXPECT(x.status == ILLUME_OK);
+    if (x.status != ILLUME_OK) continue;
+    DevMesh m;   // as the device has it
+    memcpy(&m, x.scene->s.view.meshes, sizeof(m));
+    EXPECT((m.face_normals != nullptr) == (spare == 16 * table));
+    EXPECT(m.face_normals == x.scene->s.t_meshes[0].face_normals);
+    EXPECT(g_used == need + (m.face_normals ? table : 0));
+    size_t bytes = 0;
+    EXPECT(illume_scene_upload(x.scene, &bytes) == ILLUME_OK);
+    drain();
+    EXPECT(memcmp(&m, x.scene->s.view.meshes, sizeof(m)) == 0);
+  }
+  g_limit = need - 1;
+  World x(tris, 128);
+  EXPECT(x.status == ILLUME_ERR_OOM && g_queue.empty());
+  g_limit = 0;
+}
+
 // A render whose outputs cannot be allocated, or whose passes cannot all be launched, returns
 // with nothing of it left to run: the next call's staging memory and ray counts are its own.
 static void failed_render() {
@@ -326,6 +363,7 @@ static void failed_render() {
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
+  else if (s == "face_normal_memory") face_normal_memory();
   else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);
