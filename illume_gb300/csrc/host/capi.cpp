@@ -405,6 +405,39 @@ int illume_trace_closest_device(illume_context* ctx, illume_scene* scene, const 
   return ILLUME_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// A context's kept query memory for the length of one call: out of the reach of
+// Context::release_query_memory, which an allocation in the call may ask for.
+struct KeptQueryMemory {
+  Context& c;
+  void* p;
+  size_t bytes;
+  explicit KeptQueryMemory(Context& ctx) : c(ctx), p(ctx.query_ws), bytes(ctx.query_ws_bytes) {
+    c.query_ws = nullptr;
+    c.query_ws_bytes = 0;
+  }
+  ~KeptQueryMemory() {
+    c.query_ws = p;
+    c.query_ws_bytes = bytes;
+  }
+  void* at_least(size_t need) {
+    if (bytes >= need) return p;
+    if (p) cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+    size_t want = size_t(1) << 20;
+    while (want < need) want *= 2;
+    if (cudaMalloc(&p, want) == cudaSuccess) bytes = want;
+    else { cudaGetLastError(); p = nullptr; }
+    return p;
+  }
+};
+}  // namespace
+
+extern "C" {
+
 int illume_trace_closest(illume_context* ctx, illume_scene* scene, const float* rays, int n, int intersector,
                          int bvh_kind, illume_hit* hits) {
   CHECK_ARG(ctx && scene && n >= 0 && (n == 0 || (rays && hits)), "bad argument");
@@ -415,20 +448,10 @@ int illume_trace_closest(illume_context* ctx, illume_scene* scene, const float* 
   // rays, then hits: kept memory for small calls (making and freeing device memory costs
   // more than the search of a few thousand rays), else allocated for this call
   DevBuffer own;
+  KeptQueryMemory kept(c);
   int st;
   void* mem = nullptr;
-  if (!c.budget && ray_bytes + hit_bytes <= Context::kQueryBytes) {
-    if (c.query_ws_bytes < ray_bytes + hit_bytes) {
-      if (c.query_ws) cudaFree(c.query_ws);
-      c.query_ws = nullptr;
-      c.query_ws_bytes = 0;
-      size_t want = size_t(1) << 20;
-      while (want < ray_bytes + hit_bytes) want *= 2;
-      if (cudaMalloc(&c.query_ws, want) == cudaSuccess) c.query_ws_bytes = want;
-      else { cudaGetLastError(); c.query_ws = nullptr; }
-    }
-    mem = c.query_ws;
-  }
+  if (!c.budget && ray_bytes + hit_bytes <= Context::kQueryBytes) mem = kept.at_least(ray_bytes + hit_bytes);
   if (!mem) {
     if ((st = own.alloc(&c, ray_bytes + hit_bytes)) != ILLUME_OK) return st;
     mem = own.get();

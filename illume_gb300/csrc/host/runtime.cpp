@@ -32,10 +32,18 @@ unsigned char* Context::staging() {
   return staging_;
 }
 
+bool Context::release_query_memory() {
+  if (!query_ws) return false;
+  cudaFree(query_ws);
+  query_ws = nullptr;
+  query_ws_bytes = 0;
+  return true;
+}
+
 Context::~Context() {
   if (staging_ && staging_pinned_) cudaFreeHost(staging_);
   else free(staging_);
-  if (query_ws) cudaFree(query_ws);
+  release_query_memory();
 }
 
 int DevBuffer::alloc(Context* ctx, size_t bytes) {
@@ -47,6 +55,10 @@ int DevBuffer::alloc(Context* ctx, size_t bytes) {
     return ILLUME_ERR_BUDGET;
   }
   cudaError_t e = cudaMalloc(&ptr_, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->release_query_memory()) {
+    cudaGetLastError();
+    e = cudaMalloc(&ptr_, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();   // reported here, not by a later call's check
     ptr_ = nullptr;

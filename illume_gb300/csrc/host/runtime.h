@@ -54,10 +54,12 @@ struct Context {
   static constexpr size_t kStagingBytes = size_t(1) << 20;
   unsigned char* staging();
   // Device memory kept between the host-buffer query calls (at most kQueryBytes; not under
-  // a budget, which is the caller's to spend).
+  // a budget, which is the caller's to spend). Given back when the context goes, or when one
+  // of its allocations finds no memory.
   static constexpr size_t kQueryBytes = size_t(64) << 20;
   void* query_ws = nullptr;
   size_t query_ws_bytes = 0;
+  bool release_query_memory();   // whether there was any
   Context() = default;
   Context(const Context&) = delete;
   Context& operator=(const Context&) = delete;

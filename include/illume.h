@@ -261,7 +261,9 @@ int illume_scene_load_json_string(illume_context* ctx, const char* json, const c
 int illume_scene_create(illume_context* ctx, const illume_scene_desc* desc, illume_scene** out);
 /* Fill *out with pointers into the scene's host copy (valid while the scene lives). */
 int illume_scene_describe(const illume_scene* scene, illume_scene_desc* out);
-/* Device bytes held by the scene (geometry, BVHs, textures). */
+/* Device bytes held by the scene (geometry, BVHs, textures; where it takes at most a
+ * sixteenth of the free memory and the context has no budget, 16 bytes for each triangle
+ * without vertex normals, whose face normals are then made at upload). */
 int illume_scene_device_bytes(const illume_scene* scene, size_t* out);
 /* Copies the scene's geometry to its device buffers again: triangles, vertex attributes,
  * every BVH layout, and the mesh / instance / sphere / material tables (what the
@@ -358,7 +360,10 @@ int illume_save_pfm(const float* rgb, int width, int height, const char* path);
 
 /* ---- test hooks ---- */
 /* Closest hit of n rays (8 floats each: ox, oy, oz, unused, dx, dy, dz, unused; the
- * direction is used as given) against a scene, on the device; host buffers. */
+ * direction is used as given) against a scene, on the device; host buffers. A context
+ * without a budget keeps the device memory of such calls (64 bytes a ray, up to 64 MB)
+ * for the next one; it goes with the context, or when another allocation of the context
+ * finds no memory. */
 int illume_trace_closest(illume_context* ctx, illume_scene* scene, const float* rays, int n, int intersector,
                          int bvh_kind, illume_hit* hits);
 /* Same with device pointers, on the context's stream, no synchronisation. */

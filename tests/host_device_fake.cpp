@@ -30,6 +30,7 @@ static std::vector<Op>* g_capture = nullptr;       // operations of the graph be
 static std::map<void*, size_t> g_memory;
 static size_t g_used = 0, g_limit = 0;             // g_limit 0: none
 static int g_fail_graph_launch = -1;               // countdown to a failing graph launch
+static cudaError_t g_error = cudaSuccess;          // what cudaGetLastError reports
 static int g_pass_kernels = 0;                     // kernels of passes that have run
 static std::vector<std::pair<int, int>> g_samples; // sample ranges accumulated
 
@@ -46,10 +47,14 @@ extern "C" {
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 4; return cudaSuccess; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) {
+  const cudaError_t e = g_error;
+  g_error = cudaSuccess;
+  return e;
+}
 const char* cudaGetErrorString(cudaError_t) { return "fake device error"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-  if (g_limit && g_used + n > g_limit) return cudaErrorMemoryAllocation;
+  if (g_limit && g_used + n > g_limit) return g_error = cudaErrorMemoryAllocation;
   *p = aligned_alloc(256, (n + 255) & ~(size_t)255);
   g_memory[*p] = n;
   g_used += n;
@@ -98,7 +103,7 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned lon
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete (FakeGraph*)g; return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { delete (FakeGraph*)e; return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
-  if (g_fail_graph_launch >= 0 && g_fail_graph_launch-- == 0) return cudaErrorUnknown;
+  if (g_fail_graph_launch >= 0 && g_fail_graph_launch-- == 0) return g_error = cudaErrorUnknown;
   for (const Op& f : ((FakeGraph*)e)->ops) g_queue.push_back(f);
   return cudaSuccess;
 }
@@ -360,10 +365,41 @@ static void failed_render() {
   }
 }
 
+// The device memory that small queries keep between calls is given back when an allocation
+// of the context needs it, and not while a query is using it.
+static void query_memory() {
+  World x;
+  float rays[8] = {3, 0, 0, 0, 0, 0, 1, 0};
+  illume_hit hit;
+  EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE4, &hit) == ILLUME_OK);
+  EXPECT(x.ctx->c.query_ws && hit.t == 3.0f);
+  g_limit = g_used + 4096;
+  {
+    DevBuffer b;
+    EXPECT(b.alloc(&x.ctx->c, 500000) == ILLUME_OK);
+    EXPECT(!x.ctx->c.query_ws && cudaGetLastError() == cudaSuccess);
+    // with none to give back the allocation is refused, and its error does not linger
+    DevBuffer more;
+    EXPECT(more.alloc(&x.ctx->c, 800000) == ILLUME_ERR_OOM && cudaGetLastError() == cudaSuccess);
+    // a query without memory to keep takes what it needs
+    hit.t = 0;
+    EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE4, &hit) == ILLUME_OK);
+    EXPECT(hit.t == 3.0f && !x.ctx->c.query_ws);
+  }
+  EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE4, &hit) == ILLUME_OK);
+  EXPECT(x.ctx->c.query_ws);
+  // the first 8-wide query allocates its layout while it holds the kept memory
+  g_limit = g_used;
+  EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE8, &hit) == ILLUME_ERR_OOM);
+  EXPECT(x.ctx->c.query_ws && g_memory.count(x.ctx->c.query_ws) && g_queue.empty());
+  g_limit = 0;
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
   else if (s == "face_normal_memory") face_normal_memory();
+  else if (s == "query_memory") query_memory();
   else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);
