@@ -654,12 +654,12 @@ int Scene::ensure_wide(std::string* err) {
   std::vector<int> todo;
   for (int i = 0; i < nm && i < (int)bvhs.size(); ++i)
     if (!bvhs[i].has_wide) todo.push_back(i);
-  if (todo.empty()) return ILLUME_OK;
+  if (todo.empty() && (!ctx || wide_on_device)) return ILLUME_OK;
   std::atomic<int> next{0};
   std::vector<int> sizes;
   for (int i : todo) sizes.push_back(h.mesh_num_tris[i]);
   const int nthreads = std::max(1, std::min<int>((int)todo.size(), build_threads()));
-  const int share = build_thread_share(sizes.data(), (int)sizes.size(), nthreads);
+  const int share = todo.empty() ? 1 : build_thread_share(sizes.data(), (int)sizes.size(), nthreads);
   auto work = [&]() {
     const BuildThreadShare scope(share);
     for (int k = next++; k < (int)todo.size(); k = next++) {
@@ -687,16 +687,28 @@ int Scene::ensure_wide(std::string* err) {
     device_bytes += buffers.back()->size();
     return ILLUME_OK;
   };
-  for (int i : todo) {
+  // every mesh, also where an earlier call built the layouts and found no memory for them;
+  // without memory for all of them none stays
+  const size_t had_buffers = buffers.size(), had_uploads = uploads.size(), had_bytes = device_bytes;
+  std::vector<DevMesh> table = t_meshes;
+  for (int i = 0; i < nm; ++i) {
     const MeshBvh& b = bvhs[i];
     void* pw = nullptr;
     void* pt = nullptr;
     int st = up(b.wide.data(), b.wide.size() * sizeof(WideNode), &pw);
     if (st == ILLUME_OK) st = up(b.wide_tris.data(), b.wide_tris.size() * sizeof(float4), &pt);
-    if (st != ILLUME_OK) { *err = last_error(); return st; }
-    t_meshes[i].wide = reinterpret_cast<const WideNode*>(pw);
-    t_meshes[i].wide_tris = reinterpret_cast<const float4*>(pt);
+    if (st != ILLUME_OK) {
+      *err = last_error();
+      cudaStreamSynchronize(ctx->stream);
+      buffers.resize(had_buffers);
+      uploads.resize(had_uploads);
+      device_bytes = had_bytes;
+      return st;
+    }
+    table[i].wide = reinterpret_cast<const WideNode*>(pw);
+    table[i].wide_tris = reinterpret_cast<const float4*>(pt);
   }
+  std::copy(table.begin(), table.end(), t_meshes.begin());   // (the upload list knows its address)
   // the mesh table: the source the per-render re-uploads copy from, then its device copy
   for (Upload& u : uploads)
     if (u.dst == (const void*)view.meshes) {
@@ -706,6 +718,7 @@ int Scene::ensure_wide(std::string* err) {
   ILLUME_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   ILLUME_CUDA_TRY(cudaMemcpy(const_cast<DevMesh*>(view.meshes), t_meshes.data(), sizeof(DevMesh) * (size_t)nm,
                              cudaMemcpyHostToDevice));
+  wide_on_device = true;
   return ILLUME_OK;
 }
 

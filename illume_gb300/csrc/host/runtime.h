@@ -166,6 +166,7 @@ struct Scene {
   // the device mesh table pointed at it. Renders of other layouts never wait for it.
   int ensure_wide(std::string* err);
   std::mutex wide_mu;
+  bool wide_on_device = false;             // every mesh's 8-wide layout is uploaded
 };
 
 // Process-wide cache of mesh BVH builds keyed by mesh content (runtime.cpp).

@@ -395,11 +395,33 @@ static void query_memory() {
   g_limit = 0;
 }
 
+// An 8-wide query that finds no memory for the layout uploads it when it is asked again.
+static void wide_layout_memory() {
+  World x(200);
+  float rays[8] = {3, 0, 0, 0, 0, 0, 1, 0};
+  illume_hit hit;
+  const size_t before = g_used, listed = x.scene->s.device_bytes;
+  for (size_t room : {(size_t)0, (size_t)64, (size_t)4096}) {
+    g_limit = before + 64 + room;   // (the rays and the hit take 64 bytes)
+    EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE8, &hit) == ILLUME_ERR_OOM);
+    EXPECT(g_used == before && x.scene->s.device_bytes == listed);
+  }
+  g_limit = 0;
+  EXPECT(illume_trace_closest(x.ctx, x.scene, rays, 1, ILLUME_ISECT_MT, ILLUME_BVH_WIDE8, &hit) == ILLUME_OK);
+  DevMesh m;
+  memcpy(&m, x.scene->s.view.meshes, sizeof(m));
+  const MeshBvh& b = x.scene->s.bvhs[0];
+  EXPECT(b.wide.size() > 0 && g_memory[(void*)m.wide] == b.wide.size() * sizeof(WideNode));
+  EXPECT(g_memory[(void*)m.wide_tris] == b.wide_tris.size() * sizeof(float4));
+  if (!g_failed) EXPECT(memcmp(m.wide, b.wide.data(), b.wide.size() * sizeof(WideNode)) == 0);
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
   else if (s == "face_normal_memory") face_normal_memory();
   else if (s == "query_memory") query_memory();
+  else if (s == "wide_layout_memory") wide_layout_memory();
   else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);
