@@ -521,7 +521,7 @@ int Engine::run_profiled(int depth, bool count_visits, std::vector<cudaEvent_t>&
   launch_accumulate(w, grid_acc, st);
   ILLUME_CUDA_TRY(event());
   launch_advance(w, st);
-  nl += 3;
+  nl += 2;
   ILLUME_CUDA_TRY(cudaGetLastError());
   advance_mirror();
   if (iterations) *iterations = n;

@@ -77,12 +77,13 @@ struct Engine {
   int read_row_rays(int r, unsigned long long* out);   // synchronous
   int free_rows() const;
   long long paths_in_pass() const;                      // of the next pass, from the mirror
-  // Launches of the next pass with `depth` bounces.
+  // Launches of the next pass with `depth` bounces: plan, paths (camera rays and bounces, of
+  // each half, or the path kernel alone), accumulation, advance.
   int launches_per_pass(int depth, bool nee = false) const {
-    if (path_pass(depth)) return 5;
+    if (path_pass(depth)) return 4;
     int n = 1 + (nee ? 3 : 2) * depth;
     for (int b = 2; b < depth; ++b) n += hand_over(b);
-    return 4 + (split_pass() ? 2 : 1) * n;
+    return 3 + (split_pass() ? 2 : 1) * n;
   }
   // Launches of regenerating passes with `iterations` loop iterations in all.
   static long long launches_regen(long long passes, long long iterations, bool nee = false) {

@@ -246,9 +246,9 @@ struct World {
     d.width = d.height = 16;
     return illume_scene_create(ctx, &d, &scene);
   }
-  illume_renderer* renderer(int w, int h, int spp, int per_pass = 0, int engines = 0, int estimator = 0) {
+  illume_renderer* renderer(int w, int h, int spp, int per_pass = 0, int engines = 0, int estimator = 0, int depth = 5) {
     illume_render_params p;
-    illume_render_params_default(scene, spp, 5, &p);
+    illume_render_params_default(scene, spp, depth, &p);
     p.width = w; p.height = h;
     p.samples_per_pass = per_pass; p.engines = engines; p.estimator = estimator;
     illume_renderer* r = nullptr;
@@ -416,12 +416,40 @@ static void wide_layout_memory() {
   if (!g_failed) EXPECT(memcmp(m.wide, b.wide.data(), b.wide.size() * sizeof(WideNode)) == 0);
 }
 
+// The launches a call reports are the ones its passes made.
+static void launch_counts() {
+  World x;
+  illume_render_stats st;
+  for (int depth : {0, 1, 3, 9})
+    for (int estimator = 0; estimator < 2; ++estimator)
+      // passes of the path kernel alone, of bounces with hand-over, of two halves, of engines
+      for (int k = 0; k < 4; ++k) {
+        illume_renderer* r = k == 0 ? x.renderer(64, 48, 5, 2, 0, estimator, depth)
+                             : k == 1 ? x.renderer(600, 500, 3, 1, 1, estimator, depth)
+                             : k == 2 ? x.renderer(1024, 1024, 2, 1, 0, estimator, depth)
+                                      : x.renderer(600, 500, 5, 2, 2, estimator, depth);
+        EXPECT(r);
+        if (!r) return;
+        const long long before = x.ctx->c.launches.load();
+        g_pass_kernels = 0;
+        EXPECT(illume_render_device(r, 0, &st) == ILLUME_OK);
+        EXPECT(st.kernel_launches == g_pass_kernels && x.ctx->c.launches.load() - before == g_pass_kernels);
+        illume_profile prof;
+        const long long at = x.ctx->c.launches.load();
+        g_pass_kernels = 0;
+        EXPECT(illume_renderer_profile(r, 0, &prof) == ILLUME_OK);
+        EXPECT(x.ctx->c.launches.load() - at == g_pass_kernels);
+        illume_renderer_destroy(r);
+      }
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
   else if (s == "face_normal_memory") face_normal_memory();
   else if (s == "query_memory") query_memory();
   else if (s == "wide_layout_memory") wide_layout_memory();
+  else if (s == "launch_counts") launch_counts();
   else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);
