@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128, kPathBlocks) k_paths(WaveBuffers w, int b
       ++all_rays;
       if (NEE && out.shadow) {
         VisitCount sv;
-        const HitRecord s = closest_hit<BVH_WIDE4, false, false, false, true, false, true, true, false>(
+        const HitRecord s = closest_hit<BVH_WIDE4, false, false, false, true, false, true, false, false>(
             sc, v3(out.so.x, out.so.y, out.so.z), v3(out.sd.x, out.sd.y, out.sd.z), ISECT, stack, &sv, out.sd.w);
         dropped |= sv.dropped;
         if (s.geom == -1) {

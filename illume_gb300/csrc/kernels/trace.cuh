@@ -38,7 +38,8 @@ __device__ __forceinline__ float safe_rcp(float d) {
 }
 
 // The same reciprocal from the hardware approximation (rcp.approx.ftz.f32, at most about
-// one ulp off; the clamp keeps the input normal). Used only for box tests: a relative
+// one ulp off; the clamp keeps the input normal, and up to 2^126 the result is normal too).
+// Used only for the box tests of path rays, whose directions are unit vectors: a relative
 // error e on a ray's reciprocal direction scales each axis's slab distances by (1 + e),
 // so entry and exit distances of different axes move apart by at most twice that, far
 // inside the ~8 ulp exit widening (kExitSlack), and no box that contains a hit is culled.

@@ -239,7 +239,9 @@ __global__ void __launch_bounds__(128, 8) k_trace_refill(WaveBuffers w, RenderKn
 // Shadow rays of the next-event estimator: a contribution is added to its path's
 // radiance when nothing lies within the ray's maximum distance. Occlusion needs no
 // closest hit, so the traversal stops at the first hit (binary and 4-wide layouts);
-// warps take 32 rays at a time from a counter (counters[48 + parity]).
+// warps take 32 rays at a time from a counter (counters[48 + parity]). Reciprocals are exact for
+// every trace variant (approximate ones, here and in the path kernel's occlusion search:
+// a light-sampling render 6.86 -> 6.74 ms).
 template <int KIND, int ISECT = -1>
 __global__ void __launch_bounds__(128, 8) k_shadow(WaveBuffers w, RenderKnobs k, int bounce) {
   const int parity = pass_iteration(w, bounce) & 1;
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(128, 8) k_shadow(WaveBuffers w, RenderKnobs k,
     const SceneView& sc = w.jobs[job].sc;
     VisitCount vc;
     const HitRecord h =
-        closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, KIND != BVH_WIDE8, false, KIND == BVH_WIDE4, KIND == BVH_WIDE4,
+        closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, KIND != BVH_WIDE8, false, KIND == BVH_WIDE4, false,
                     false, ISECT>(sc, v3(so.x, so.y, so.z), v3(sd.x, sd.y, sd.z), k.isect, stack, &vc, sd.w);
     if (vc.dropped) atomicOr(w.counters + kCounterStackDrops, 1);
     if (h.geom == -1) {
@@ -430,8 +432,9 @@ __global__ void __launch_bounds__(128) k_trace_sm(WaveBuffers w, const SceneView
 // longest search, so rays that do not fill the device are spread over more warps. Blocks
 // of 64 give a finished block's place to the next one sooner than blocks of 128.
 // 3M unordered rays on 16 meshes (500k triangles): 5.19 ms with the compiler's registers,
-// exact reciprocals and instances in index order, 2.32 ms with the default trace kernel's
-// settings. FEW: at most 102 registers for batches that do not fill the device at 64, where
+// exact reciprocals and instances in index order, 2.43 ms with the default trace kernel's
+// settings but for the reciprocals (2.39 with its approximate ones: a query's direction may
+// have any length, and above 2^126 they flush to zero, which loses hits). FEW: at most 102 registers for batches that do not fill the device at 64, where
 // latency counts (1,000 rays 192 -> 41 us, 20,000 on one mesh 74 -> 66, 100,000 97 -> 90;
 // at 64 registers 45, 82 and 109).
 template <int KIND, int ISECT = -1, bool FEW = false>
@@ -444,9 +447,9 @@ __global__ void __launch_bounds__(64, KIND == BVH_WIDE4 ? (FEW ? 10 : 16) : 1)
   if (lane >= width || first + lane >= n) return;
   const size_t i = (size_t)(first + lane);
   const float4 a = rays[2 * i], b = rays[2 * i + 1];
-  // the binary and 4-wide layouts are searched with the box arithmetic and traversal order
-  // of their default trace kernels
-  const HitRecord h = closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, false, false, W4, W4, W4, ISECT>(
+  // the binary and 4-wide layouts are searched with the box arithmetic (reciprocals apart) and
+  // traversal order of their default trace kernels
+  const HitRecord h = closest_hit<KIND, false, KIND == BVH_BINARY, KIND == BVH_BINARY, false, false, W4, false, W4, ISECT>(
       sc, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), isect, stack);
   illume_hit o;
   o.t = h.t;
