@@ -139,14 +139,18 @@ int Renderer::init(std::string* err) {
   RenderKnobs knobs = render_knobs(p);
   knobs.overlap = nengines > 1;
   // A pass of one engine, left to choose, runs as two halves side by side from 1M paths on in
-  // a scene without an environment: there most paths go on for many bounces, and each bounce's
-  // last rays leave much of the device to the other half. Device ms, whole / halves: Cornell box
-  // of 1.05M paths 0.500 / 0.441, 2.1M 0.914 / 0.835, 1024x768 x 4 samples 1.476 / 1.350, watertight 2.1M 1.048 / 0.907, next-event 1.998 / 1.846; subsurface
-  // 1.2M 4.49 / 3.97, 2.8M 11.34 / 10.66, 4.0M 15.17 / 14.21; two engines of 0.26M paths
-  // each lose 10 to 30%. Under a sky most rays leave early and
-  // halves run from 4% faster to 14% slower (2.1M paths: ground 1.49 / 1.53, textured 2.06 /
-  // 2.20, 16 meshes 1.98 / 2.01, mixed 1.33 / 1.36).
-  eng.halves = p.engines == 0 && nengines == 1 && scene->view.env_tex < 0 && paths_kernel_for(knobs) && p.queue_slots == 0;
+  // a room without an environment: there most paths go on for many bounces, and each
+  // bounce's last rays leave much of the device to the other half. Passes of 1.05M to 4M
+  // paths, whole / halves, device time:
+  //   five and six walls around a shape, 16 meshes, a mixed or a textured scene: 0.99 to 1.17
+  //   (36 passes, mean 1.06); Cornell box 1.08 to 1.16 (1.05M paths 0.585 / 0.503 ms, 4.1M
+  //   2.02 / 1.78), a body of a medium in it 1.00 to 1.07 (4.1M 12.56 / 11.84)
+  //   four walls, or none and a lamp overhead: 0.85 to 1.17, textured scenes 0.85 to 0.99 (1.3M
+  //   paths 1.56 / 1.81 ms), one shape on the ground 0.93 to 1.02
+  // Two engines of 0.26M paths each lose 10 to 30%. Under a sky most rays leave early too:
+  // 0.86 to 1.04 (2.1M paths: ground 1.49 / 1.53, textured 2.06 / 2.20).
+  eng.halves = p.engines == 0 && nengines == 1 && scene->room && scene->view.env_tex < 0 && paths_kernel_for(knobs) &&
+               p.queue_slots == 0;
   if ((st = eng.init(ctx, 1, per_pass * npix, knobs, err, p.queue_slots, p.regen_threshold)) != ILLUME_OK)
     return st;
   JobDesc row = job_row(*scene, p, acc);

@@ -440,6 +440,53 @@ int Scene::build_host(std::string* err) {
   return ILLUME_OK;
 }
 
+// Whether the scene is a room: at least five of the six faces of its bounding box are walls,
+// nine tenths covered by triangles that lie in the face (within a hundredth of the box) and
+// neither shine nor let light through. Paths go on in a room until their throughput or
+// their depth ends, whatever stands in it. (Walls are few triangles: a mesh of more than
+// 4,096 is taken for something that stands in the room, so this costs next to nothing.)
+static bool closed_room(const SceneHost& h, const std::vector<DevInstance>& inst, const std::vector<DevSphere>& spheres) {
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  auto cover = [&](int a, double l, double u) {
+    lo[a] = std::min(lo[a], l);
+    hi[a] = std::max(hi[a], u);
+  };
+  for (const DevInstance& in : inst)
+    for (int a = 0; a < 3 && in.lo[0] <= in.hi[0]; ++a) cover(a, in.lo[a], in.hi[a]);
+  for (const DevSphere& s : spheres) {
+    const float c[3] = {s.cx, s.cy, s.cz};
+    for (int a = 0; a < 3; ++a) cover(a, c[a] - fabs(s.r), c[a] + fabs(s.r));
+  }
+  double area[6] = {};   // covered, of faces lo x, hi x, lo y, ...
+  for (size_t i = 0; i < inst.size(); ++i) {
+    const int m = inst[i].mesh, type = h.mat_type[inst[i].material];
+    if (h.mesh_num_tris[m] > 4096 || type == MAT_EMISSIVE || type == MAT_REFRACTIVE || type == MAT_ROUGHREFRACTIVE) continue;
+    const float* M = h.inst_mat.data() + 12 * i;
+    const float* P = h.positions.data() + 3 * (size_t)h.mesh_vertex_offset[m];
+    const int* T = h.tris.data() + 3 * (size_t)h.mesh_tri_offset[m];
+    for (int t = 0; t < h.mesh_num_tris[m]; ++t) {
+      double v[3][3];
+      for (int k = 0; k < 3; ++k) {
+        const float* p = P + 3 * (size_t)T[3 * t + k];
+        for (int a = 0; a < 3; ++a) v[k][a] = M[4 * a] * p[0] + M[4 * a + 1] * p[1] + M[4 * a + 2] * p[2] + M[4 * a + 3];
+      }
+      for (int f = 0; f < 6; ++f) {
+        const int a = f / 2, b = (a + 1) % 3, c = (a + 2) % 3;
+        const double plane = f & 1 ? hi[a] : lo[a], near = 0.01 * (hi[a] - lo[a]);
+        if (!(fabs(v[0][a] - plane) <= near && fabs(v[1][a] - plane) <= near && fabs(v[2][a] - plane) <= near)) continue;
+        area[f] += 0.5 * fabs((v[1][b] - v[0][b]) * (v[2][c] - v[0][c]) - (v[1][c] - v[0][c]) * (v[2][b] - v[0][b]));
+      }
+    }
+  }
+  int walls = 0;
+  for (int f = 0; f < 6; ++f) {
+    const int b = (f / 2 + 1) % 3, c = (f / 2 + 2) % 3;
+    const double face = (hi[b] - lo[b]) * (hi[c] - lo[c]);
+    walls += face > 0.0 && area[f] >= 0.9 * face;
+  }
+  return walls >= 5;
+}
+
 int Scene::build_and_upload(std::string* err) {
   const SceneHost& h = host;
   const int nm = h.num_meshes();
@@ -524,6 +571,7 @@ int Scene::build_and_upload(std::string* err) {
     spheres[i].r = h.sphere_center_radius[4 * i + 3];
     spheres[i].material = h.sphere_material[i];
   }
+  room = closed_room(h, inst, spheres);
   const int nmat = h.num_materials();
   std::vector<DevMaterial>& mats = t_materials;
   mats.assign(nmat, DevMaterial{});

@@ -188,9 +188,10 @@ typedef struct {
                                * turns on the passes of a call, so that one pass's last bounces
                                * overlap the next passes; 0 = for a pass of 4M paths or more one
                                * per 16M paths, 2 to 4, else 1 (a pass of 1M paths or more in a
-                               * scene without an environment then runs as two halves side by
-                               * side on that engine; not with 1); at most 16 and at most the
-                               * samples per pass.
+                               * room without an environment, a scene most of whose bounding
+                               * box is walls, then runs as two halves side by side on that
+                               * engine; not with 1); at most 16 and at most the samples per
+                               * pass.
                                * The image does not depend on it. The server ignores it
                                * (ILLUME_SERVER_LANES). */
   /* Path regeneration (no counterpart in the reference, whose passes hold one sample of
