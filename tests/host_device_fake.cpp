@@ -419,6 +419,7 @@ static void wide_layout_memory() {
 // The launches a call reports are the ones its passes made.
 static void launch_counts() {
   World x;
+  x.scene->s.room = true;   // (a strip of triangles otherwise, whose passes run whole)
   illume_render_stats st;
   for (int depth : {0, 1, 3, 9})
     for (int estimator = 0; estimator < 2; ++estimator)
