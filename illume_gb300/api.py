@@ -13,7 +13,6 @@ from __future__ import annotations
 
 import ctypes
 import os
-import weakref
 from typing import Optional
 
 import numpy as np
@@ -22,24 +21,34 @@ from . import _capi as C
 from .scenedata import SceneData
 
 
+def _close(handle: ctypes.c_void_p, destroy) -> None:
+    if handle:
+        destroy(handle)
+        handle.value = None
+
+
 class Context:
     """One device and one CUDA stream. Closing a context first closes the servers,
     renderers and scenes made with it (newest first), which must not outlive it."""
 
     def __init__(self, device: int = 0, hbm_budget_bytes: int = 0):
         self.handle = ctypes.c_void_p()
-        self._children = []
+        self._children, self._live = [], 0
         C.check(C.lib().illume_context_create(device, hbm_budget_bytes, ctypes.byref(self.handle)))
 
-    def _adopt(self, obj):
-        self._children.append(weakref.ref(obj))
+    # Children are known by their handles, not by references to the objects: when a context
+    # and its children are collected as one garbage cycle, weak references to them are gone
+    # before the first of them is finalised, and that may be the context.
+    def _adopt(self, handle, destroy):
+        if len(self._children) >= 2 * self._live + 16:
+            self._children = [c for c in self._children if c[0]]
+            self._live = len(self._children)
+        self._children.append((handle, destroy))
 
     def close(self):
         if self.handle:
-            for ref in reversed(self._children):
-                obj = ref()
-                if obj is not None:
-                    obj.close()
+            for handle, destroy in reversed(self._children):
+                _close(handle, destroy)
             self._children = []
             C.lib().illume_context_destroy(self.handle)
             self.handle = ctypes.c_void_p()
@@ -67,7 +76,7 @@ class HostScene:
     def __init__(self, ctx: Context, handle: ctypes.c_void_p):
         self.ctx = ctx
         self.handle = handle
-        ctx._adopt(self)
+        ctx._adopt(self.handle, C.lib().illume_scene_destroy)
 
     @staticmethod
     def from_json_file(ctx: Context, path: str, base_dir: Optional[str] = None) -> "HostScene":
@@ -127,9 +136,7 @@ class HostScene:
         return {k: a[k].copy() for k in ("t", "u", "v", "inst", "prim", "sphere")}
 
     def close(self):
-        if self.handle:
-            C.lib().illume_scene_destroy(self.handle)
-            self.handle = ctypes.c_void_p()
+        _close(self.handle, C.lib().illume_scene_destroy)
 
     def __del__(self):
         try:
@@ -173,7 +180,7 @@ class Renderer:
         self.params = p
         self.handle = ctypes.c_void_p()
         C.check(C.lib().illume_renderer_create(ctx.handle, scene.handle, ctypes.byref(p), ctypes.byref(self.handle)))
-        ctx._adopt(self)
+        ctx._adopt(self.handle, C.lib().illume_renderer_destroy)
 
     def get_width(self) -> int:
         return C.lib().illume_renderer_get_width(self.handle)
@@ -214,9 +221,7 @@ class Renderer:
         return dict(mean=m, sum=s, sumsq=s2, rgb8=r8)
 
     def close(self):
-        if self.handle:
-            C.lib().illume_renderer_destroy(self.handle)
-            self.handle = ctypes.c_void_p()
+        _close(self.handle, C.lib().illume_renderer_destroy)
 
     def __del__(self):
         try:
@@ -239,7 +244,7 @@ class Server:
         self.ctx = ctx
         self.handle = ctypes.c_void_p()
         C.check(C.lib().illume_server_create(ctx.handle, hbm_budget_bytes, max_jobs_in_flight, ctypes.byref(self.handle)))
-        ctx._adopt(self)
+        ctx._adopt(self.handle, C.lib().illume_server_destroy)
         self._npix = {}
         names = {"path_capacity": C.SERVER_PATH_CAPACITY, "passes_per_step": C.SERVER_PASSES_PER_STEP,
                  "autotune": C.SERVER_AUTOTUNE, "trace_variant": C.SERVER_TRACE_VARIANT, "lanes": C.SERVER_LANES,
@@ -291,9 +296,7 @@ class Server:
         return s
 
     def close(self):
-        if self.handle:
-            C.lib().illume_server_destroy(self.handle)
-            self.handle = ctypes.c_void_p()
+        _close(self.handle, C.lib().illume_server_destroy)
 
     def __del__(self):
         try:
