@@ -134,8 +134,9 @@ __device__ __forceinline__ int ray_bounce(const WaveBuffers& w, int parity, int 
 static constexpr int kDefaultRayGroup = 16;
 
 // The path kernel (paths.cu): blocks of 128 per SM (at most 128 registers, no spills; 5 and
-// 6 blocks spill: a 64x48 render 7-19% slower, a 1280x720 sample 5%), the largest pass that runs as one launch of it, and
-// the rays at which a larger pass hands the rest of its paths over.
+// 6 blocks spill: a 64x48 render 7-19% slower, a 1280x720 sample 5%), the largest pass that
+// runs as one launch of it, and the rays at which a larger pass hands the rest of its paths
+// over.
 // Pass of 12 bounces, ms, wavefront with hand-over / one path-kernel launch, by paths:
 //              2^14        2^16        2^17        2^18        2^19        2^20
 //   Cornell    .21 / .12   .22 / .14   .27 / .19   .33 / .32   .48 / .56   .80 / 1.06
@@ -143,9 +144,11 @@ static constexpr int kDefaultRayGroup = 16;
 //   medium     .38 / .25   .47 / .35   .60 / .52   .93 / .97  1.41 / 1.84 2.14 / 3.58
 //   NEE        .48 / .28   .64 / .45   .75 / .61   .96 / 1.01 1.20 / 1.76 1.63 / 3.24
 // The wavefront runs lanes of one event class together, which pays once a bounce fills the
-// device several times over (311,296 lanes at 64 registers). Hand-over at 2^16 / 2^17 /
-// 2^18 / 2^19 rays: textured scene 2.54 / 2.19 / 2.21 / 2.37 ms, light sampling 7.02 /
-// 7.17 / 7.18 / 7.59, 16 large meshes 5.65 / 5.63 / 5.62 / 5.89.
+// device more than once (155,648 lanes at 64 registers on 152 SMs). One limit for every
+// scene: at 2^18 paths a medium and light sampling give away 4 to 5% of a pass, and beyond
+// it mixed scenes 4 to 23%; which scene is which is not known before its paths have run.
+// Hand-over at 2^16 / 2^17 / 2^18 / 2^19 rays: textured scene 2.54 / 2.19 / 2.21 / 2.37 ms,
+// light sampling 7.02 / 7.17 / 7.18 / 7.59, 16 large meshes 5.65 / 5.63 / 5.62 / 5.89.
 // Where passes of other tables run beside it the path kernel holds registers they could
 // use: there a larger pass hands over at 3 * 2^15 rays, 32 to a warp (light sampling 6.90
 // -> 6.68 ms, a textured render of 6M paths 5.00 -> 4.83, instances 3.36 -> 3.23, served
@@ -159,10 +162,15 @@ static constexpr int kPathTailOverlap = 3 << 15;
 // Settings shared by every job of a table (they select kernel instances).
 struct RenderKnobs {
   int isect;           // illume_intersector
-  int bvh_kind;        // BVH_BINARY or BVH_WIDE8
+  int bvh_kind;        // BvhKind
   int trace_variant;   // see trace_kernel_ptr
   int shade_variant;   // see shade_kernel_ptr
-  int overlap;         // 1: passes of other tables run beside this table's (launch_trace)
+  // 1: passes of other tables may run beside this table's (launch_trace, launch_paths): set for
+  // a renderer of several engines and a server of several lanes, whether or not the others
+  // have work. A lone request on a server of four lanes (64x48 to 1024x768, six scenes,
+  // both tests) takes these settings too: 1.02 to 3.6 times as fast as before they and the
+  // path kernel were there.
+  int overlap;
 };
 
 int kernel_grid_blocks(const void* fn, int block, int device);

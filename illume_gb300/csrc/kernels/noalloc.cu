@@ -106,8 +106,8 @@ extern "C" int illume_render_noalloc(illume_context* ctx, illume_scene* scene, c
     return ILLUME_ERR_UNSUPPORTED;
   }
   if (p.samples_per_pass > 1 || p.engines > 1 || p.queue_slots > 0) {
-    set_error("illume_render_noalloc renders one sample per pass on one engine without path regeneration "
-              "(samples_per_pass and engines must be 0 or 1, queue_slots 0)");
+    set_error("illume_render_noalloc chooses the samples of a pass itself and runs on one engine without path "
+              "regeneration (samples_per_pass and engines must be 0 or 1, queue_slots 0)");
     return ILLUME_ERR_UNSUPPORTED;
   }
   const RenderKnobs k = render_knobs(p);

@@ -318,7 +318,11 @@ int illume_render_device(illume_renderer* r, int accumulate, illume_render_stats
 int illume_renderer_read(illume_renderer* r, float* out_mean, double* out_sum, double* out_sumsq, uint8_t* out_rgb8);
 
 /* Per-stage timing of one wavefront pass (samples_per_pass samples of every pixel),
- * launched kernel by kernel with CUDA events on the context stream. With count_visits,
+ * launched kernel by kernel with CUDA events on the context stream: every bounce through
+ * the stages, one after another. A render runs otherwise where that is faster: with the
+ * default layout and trace variant a pass of up to 2^18 paths, and the last paths of a
+ * larger one, in one kernel, two halves of a pass or a bounce's occlusion rays beside other
+ * launches; the stage times here then are not parts of the render's time. With count_visits,
  * the pass runs an instrumented trace kernel that counts node fetches and triangle
  * tests (its timings are then not representative). Accumulates into the renderer like
  * a progressive call. */
