@@ -222,7 +222,7 @@ int Renderer::enqueue(bool accumulate, Call* call) {
   int s;
   for (int e = 0; e < nengines; ++e)
     if ((s = engine(e).write_pass_state(0)) != ILLUME_OK) return s;
-  call->npasses = spp > 0 ? (spp + per_pass - 1) / per_pass : 0;
+  call->npasses = spp / per_pass + (spp % per_pass != 0);   // (spp may be the largest int)
   int64_t before = 0;
   for (int e = 0; e < nengines; ++e) before += engine(e).launches;
   ILLUME_CUDA_TRY(cudaEventRecord(ev0, st));

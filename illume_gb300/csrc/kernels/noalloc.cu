@@ -188,7 +188,7 @@ extern "C" int illume_render_noalloc(illume_context* ctx, illume_scene* scene, c
   const int sms = ctx->c.sm_count > 0 ? ctx->c.sm_count : 1;
   const int grid_small = std::max(1, std::min(((int)npix + 255) / 256, sms * 8));
   k_noalloc_begin<<<grid_small, 256, 0, st>>>(w.counters, w.rays, w.visits, w.jobs, row, d_sum, (int)npix);
-  const int npasses = (p.spp + per_pass - 1) / per_pass;
+  const int npasses = p.spp / per_pass + (p.spp % per_pass != 0);   // (spp may be the largest int)
   for (int s = 0; s < npasses; ++s) {
     launch_plan(w, st);
     if (paths) {

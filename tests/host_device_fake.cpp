@@ -147,7 +147,7 @@ void launch_accumulate(const WaveBuffers& w, int, cudaStream_t) {
   push([w] {
     for (int j = 0; j < w.njobs; ++j)
       if (w.jobs[j].nsamples > 0) {
-        w.jobs[j].rays += kRaysPerSample * w.jobs[j].nsamples;
+        w.jobs[j].rays += (unsigned long long)kRaysPerSample * w.jobs[j].nsamples;
         g_samples.emplace_back(w.jobs[j].sample_base, w.jobs[j].sample_base + w.jobs[j].nsamples);
       }
   });
@@ -444,6 +444,24 @@ static void launch_counts() {
       }
 }
 
+// The largest sample count renders all its samples.
+static void largest_sample_count() {
+  World x;
+  const int spp = 0x7fffffff;
+  illume_renderer* r = x.renderer(16, 16, spp, 4000000, 1);
+  EXPECT(r);
+  if (!r) return;
+  g_samples.clear();
+  EXPECT(illume_render_device(r, 0, nullptr) == ILLUME_OK);
+  long long n = 0;
+  for (auto& s : g_samples) {
+    EXPECT(s.first == n);
+    n = s.second;
+  }
+  EXPECT(n == spp);
+  illume_renderer_destroy(r);
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "pass_state") pass_state();
@@ -451,6 +469,7 @@ int main(int argc, char** argv) {
   else if (s == "query_memory") query_memory();
   else if (s == "wide_layout_memory") wide_layout_memory();
   else if (s == "launch_counts") launch_counts();
+  else if (s == "largest_sample_count") largest_sample_count();
   else if (s == "failed_render") failed_render();
   else { printf("unknown scenario\n"); return 2; }
   if (g_failed) printf("%d expectations failed\n", g_failed);

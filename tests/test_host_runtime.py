@@ -31,7 +31,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["pass_state", "failed_render", "face_normal_memory",
-                                      "query_memory", "wide_layout_memory", "launch_counts"])
+                                      "query_memory", "wide_layout_memory", "launch_counts", "largest_sample_count"])
 def test_host_runtime(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
